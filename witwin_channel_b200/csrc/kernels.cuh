@@ -13,6 +13,7 @@
 
 #include "em.cuh"
 #include "paths.cuh"
+#include "shaft.cuh"
 #include "solve.h"
 #include "utd.cuh"
 
@@ -23,6 +24,7 @@ constexpr int kCompBlock = kWarpsPerBlock * 32;
 constexpr int kSplitWarps = 8;                 // reflection/diffraction: one tile per block,
 constexpr int kSplitBlock = kSplitWarps * 32;  // its candidates interleaved over 8 warps
 constexpr int kQueueCap = 64;
+constexpr int kCandCap = 64;  // reflection candidates listed per round and warp
 constexpr unsigned kFull = 0xffffffffu;
 
 // ------------------------------------------------------------------ common
@@ -98,6 +100,27 @@ WCB_D bool tile_cell(const MainParams& p, long long tile_global, int lane, int* 
     if (r64 >= p.num_rx) return false;
     *r = int(r64);
     return true;
+}
+
+// Reflection and diffraction give a tile a group of `warps` of the block's
+// kSplitWarps warps (1, 2, 4 or 8); a block holds kSplitWarps / warps tiles.
+struct TileGroup {
+    int warps, index, rank;  // warps per tile, group within the block, this warp within the group
+    long long tile;
+    WCB_D void sync() const {
+        if (warps == 1) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(index + 1), "r"(warps * 32) : "memory");
+    }
+};
+
+WCB_D TileGroup tile_group(int warps) {
+    const int warp = threadIdx.x >> 5;
+    TileGroup g;
+    g.warps = warps;
+    g.index = warp / warps;
+    g.rank = warp - g.index * warps;
+    g.tile = (long long)blockIdx.x * (kSplitWarps / warps) + g.index;
+    return g;
 }
 
 WCB_D unsigned lanemask_lt() {
@@ -237,6 +260,149 @@ __global__ void __launch_bounds__(kCompBlock) k_los_trans(MainParams p) {
 }
 
 // ------------------------------------------------------------------ reflection
+// Axis-aligned bounds of a tile's receivers.
+struct TileBounds {
+    float lo[3], hi[3];
+};
+
+// Bounds of the warp's active receivers (every lane gets them; a tile has at
+// least one).
+WCB_D TileBounds tile_bounds(V3<float> R, bool active) {
+    const float inf = __int_as_float(0x7f800000);
+    TileBounds b;
+    const float v[3] = {R.x, R.y, R.z};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        b.lo[k] = active ? v[k] : inf;
+        b.hi[k] = active ? v[k] : -inf;
+        for (int o = 16; o > 0; o >>= 1) {
+            b.lo[k] = fminf(b.lo[k], __shfl_xor_sync(0xffffffffu, b.lo[k], o));
+            b.hi[k] = fmaxf(b.hi[k], __shfl_xor_sync(0xffffffffu, b.hi[k], o));
+        }
+    }
+    return b;
+}
+
+// One bounce of the tile test: may a point within [lo, hi] have its back
+// projection through (plane, image) inside the group's box?  On true, [lo, hi]
+// become bounds of those back projections.  FP32, and conservative against the
+// FP64 solve: x(R), the point where the line from the image to R meets the
+// plane, is a projective map of R, so while d = n.(image - R) keeps one sign
+// over the bounds every x(R) lies in the hull of the corners' points.  A
+// crossing strictly between image and R needs them on opposite sides of the
+// plane, which the corners decide too (n.R is linear).  With S = |R| + |image|
+// + |offset| (1-norms, the largest over the corners) FP32 forms n.R - off and
+// n.image - off within 4e-7 S and d within 1e-6 S, so t = (off - n.R) / d is off
+// by at most 3e-6 S (1 + |t|) / |d| and x by that times |image - R|, which
+// widens the bounds; a d below 1e-5 S (a sign FP32 cannot tell) keeps the whole
+// group box.
+WCB_D bool project_bounds(float nx, float ny, float nz, float off, float ix, float iy, float iz, const float* bx,
+                          float (&lo)[3], float (&hi)[3]) {
+    const float h_img = nx * ix + ny * iy + nz * iz - off;
+    const float inf = __int_as_float(0x7f800000);
+    float size = 0.f, d_min = inf, d_max = -inf, t_abs = 0.f, len = 0.f, h_min = inf, h_max = -inf;
+    float xlo[3] = {inf, inf, inf}, xhi[3] = {-inf, -inf, -inf};
+    const int layers = lo[2] < hi[2] ? 2 : 1;
+#pragma unroll 1
+    for (int z = 0; z < layers; ++z) {
+        const float Rz = z == 0 ? lo[2] : hi[2];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float Rx = (q & 1) ? hi[0] : lo[0];
+            const float Ry = (q & 2) ? hi[1] : lo[1];
+            const float h = nx * Rx + ny * Ry + nz * Rz - off;
+            const float d = h_img - h;
+            const float t = __fdividef(-h, d);
+            const float ox = ix - Rx, oy = iy - Ry, oz = iz - Rz;
+            const float x[3] = {Rx + ox * t, Ry + oy * t, Rz + oz * t};
+            h_min = fminf(h_min, h);
+            h_max = fmaxf(h_max, h);
+            d_min = fminf(d_min, d);
+            d_max = fmaxf(d_max, d);
+            t_abs = fmaxf(t_abs, fabsf(t));
+            size = fmaxf(size, fabsf(Rx) + fabsf(Ry) + fabsf(Rz));
+            len = fmaxf(len, fmaxf(fabsf(ox), fmaxf(fabsf(oy), fabsf(oz))));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                xlo[k] = fminf(xlo[k], x[k]);
+                xhi[k] = fmaxf(xhi[k], x[k]);
+            }
+        }
+    }
+    size += fabsf(ix) + fabsf(iy) + fabsf(iz) + fabsf(off);
+    // every point on the image's side of the plane
+    const float h_tol = 1e-6f * size;
+    if ((h_img > h_tol && h_min > h_tol) || (h_img < -h_tol && h_max < -h_tol)) return false;
+    const float d_abs = d_min > 0.f ? d_min : (d_max < 0.f ? -d_max : 0.f);
+    float pad = inf;
+    if (d_abs > 1e-5f * size) {
+        const float xs = fmaxf(fabsf(xlo[0]), fabsf(xhi[0])) + fmaxf(fabsf(xlo[1]), fabsf(xhi[1])) +
+                         fmaxf(fabsf(xlo[2]), fabsf(xhi[2]));
+        pad = 1e-2f + 1e-5f * xs + 4e-6f * size * (1.f + t_abs) * len / d_abs;
+    }
+    bool keep = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = pad < inf ? fmaxf(bx[k], xlo[k] - pad) : bx[k];
+        hi[k] = pad < inf ? fminf(bx[3 + k], xhi[k] + pad) : bx[3 + k];
+        keep = keep && !(lo[k] > hi[k]);
+    }
+    return keep;
+}
+
+// False only when no receiver within the tile's bounds can have its FP64 back
+// projection through chain c (depth d) inside every group's box: the bounds go
+// back bounce by bounce, each cut to its group's box.
+WCB_D bool tile_may_reflect(const MainParams& p, const TileBounds& b, long long base, int c, int d) {
+    float lo[3] = {b.lo[0], b.lo[1], b.lo[2]}, hi[3] = {b.hi[0], b.hi[1], b.hi[2]};
+    const float4 pl = __ldg(p.chain_pre + (base + c) * 2);
+    const float4 im = __ldg(p.chain_pre + (base + c) * 2 + 1);
+    if (!project_bounds(pl.x, pl.y, pl.z, pl.w, im.x, im.y, im.z, p.sc.group_box + 6 * __float_as_int(im.w), lo, hi))
+        return false;
+    const long long row = base + (long long)c * d;
+    for (int k = d - 2; k >= 0; --k) {
+        const double* q = p.chain_planes + (row + k) * 4;
+        const double* i = p.chain_images + (row + k) * 3;
+        if (!project_bounds(float(q[0]), float(q[1]), float(q[2]), float(q[3]), float(i[0]), float(i[1]), float(i[2]),
+                            p.sc.group_box + 6 * p.chain_groups[row + k], lo, hi))
+            return false;
+    }
+    return true;
+}
+
+// Does one triangle block the last leg (hit on the last plane -> receiver) of
+// chain c for every receiver of the tile?  The legs lie on the lines from the
+// last image, so the shaft is that image's pencil through the tile, and only
+// occluders on the receivers' side of the plane count.
+WCB_D bool last_leg_blocked(const MainParams& p, const TileBounds& b, long long base, int c, int* stack) {
+    const float4 pl = __ldg(p.chain_pre + (base + c) * 2);
+    const float4 im = __ldg(p.chain_pre + (base + c) * 2 + 1);
+    const V3<float> mid = v3(0.5f * (b.lo[0] + b.hi[0]), 0.5f * (b.lo[1] + b.hi[1]), 0.5f * (b.lo[2] + b.hi[2]));
+    const V3<float> half = v3(0.5f * (b.hi[0] - b.lo[0]), 0.5f * (b.hi[1] - b.lo[1]), 0.5f * (b.hi[2] - b.lo[2]));
+    const V3<float> img = v3(im.x, im.y, im.z), n = v3(pl.x, pl.y, pl.z);
+    const float h = dot(n, mid) - pl.w, h_img = dot(n, img) - pl.w;
+    const float size = fmaxf(norm1(mid) + norm1(half), norm1(img));
+    const float tol = 1e-4f + 2e-5f * size;
+    if (!((h > tol && h_img < -tol) || (h < -tol && h_img > tol))) return false;
+    const V3<float> hit = mid + (img - mid) * (h / (h - h_img));
+    Shaft s;
+    s.a[0] = s.a[1] = img;
+    s.na = 1;
+    for (int k = 0; k < 3; ++k) {
+        s.lo[k] = b.lo[k];
+        s.hi[k] = b.hi[k];
+    }
+    s.size = size;
+    s.pn[0] = n.x;
+    s.pn[1] = n.y;
+    s.pn[2] = n.z;
+    s.poff = pl.w;
+    s.side = h > 0.f ? 1.f : -1.f;
+    Ignore ig = ignore_none();
+    ig.g0 = __float_as_int(im.w);
+    return shaft_blocked(p.sc, hit, mid, ig, s, stack);
+}
+
 // Per-warp shared layout: queue A (3 ints/item), queue B (3 + 5 ints/item),
 // queue F (3 + 5 ints/item), contribution buffer (32 items x NF x 3 floats).
 template <int NF>
@@ -298,15 +464,28 @@ WCB_D int queue_pop_faces(int* q, int* qfaces, int size, int n, int lane) {
 // the same kind of work: most candidates are blocked on their first segment
 // and leave after one traversal instead of idling while a visible path of
 // the same batch traces its remaining segments and its field.
+//
+// Bound by instruction issue and fetch (ncu on the 64-box canyon, 256^2 cells:
+// 32 % issue, 4.1 no-instruction stalls per issue; DRAM below 1 %).  Most of
+// the work was on candidates that no receiver of a tile has: of 1.71 M (tile,
+// candidate) pairs the last bounce's box alone left 222 k (6.7 M FP64 back
+// projections), all bounces' boxes leave 61 k and the blocked last legs 31 k
+// (0.77 M).  Testing the receiver's leg first takes the visibility segments of
+// what is left from 1.8 to 1.3 per candidate.  Before and after, on one B200:
+// canyon 1.25 -> 0.80 ms, four-transmitter batch 15.4 -> 8.0 ms, 2048-box city
+// (1024^2 cells, depth 5) 167 -> 25-30 ms, a 90 x 70 town with 25,760
+// exhaustive chains 4.0 -> 0.6 ms.
 template <typename T, int NF>
-__global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect(MainParams p, int stack_depth) {
+__global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect(MainParams p, int stack_depth,
+                                                                                           int tile_warps) {
     extern __shared__ int smem[];
     int* stack = smem;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     ReflShared<NF>* sh = reinterpret_cast<ReflShared<NF>*>(smem + stack_depth * kSplitBlock) + warp;
     float* red = reinterpret_cast<float*>(reinterpret_cast<ReflShared<NF>*>(smem + stack_depth * kSplitBlock) + kSplitWarps);
-    const long long tile = blockIdx.x;
+    const TileGroup grp = tile_group(tile_warps);
+    const long long tile = grp.tile;
     int t = 0, r = 0;
     const bool active = tile_cell(p, tile, lane, &t, &r);
     // the whole warp shares the tile's transmitter
@@ -436,8 +615,8 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
             ok = !segment_blocked<T>(sc, cast3<T>(a), cast3<T>(b), ig, stack, err);
         }
         qb = queue_pop_faces(sh->qb, sh->qbf, qb, n, lane);
-        qb = queue_push_faces(sh->qb, sh->qbf, qb, ok && s < d, it_lane, c, d | ((s + 1) << 4), faces);
-        qf = queue_push_faces(sh->qf, sh->qff, qf, ok && s == d, it_lane, c, d, faces);
+        qb = queue_push_faces(sh->qb, sh->qbf, qb, ok && s > 0, it_lane, c, d | ((s - 1) << 4), faces);
+        qf = queue_push_faces(sh->qf, sh->qff, qf, ok && s == 0, it_lane, c, d, faces);
     };
 
     // stage A: FP64 back projection + containment for up to 32 items; the
@@ -473,58 +652,123 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
             }
         }
         qa = queue_pop(sh->qa, qa, n, lane);
-        qb = queue_push_faces(sh->qb, sh->qbf, qb, ok, it_lane, c, d, faces);
+        qb = queue_push_faces(sh->qb, sh->qbf, qb, ok, it_lane, c, d | (d << 4), faces);
     };
 
     if ((p.components & 2) && sc.num_faces > 0) {
-        // One loop drives the stages so each is inlined once.  Each pass runs
-        // one step, full batches first and the latest stage first: F, then B,
-        // then A, then the next candidate into queue A; partial batches only
-        // once nothing upstream can fill them.  A stage runs only while the
-        // queues it feeds hold fewer than 32 items, so no queue exceeds 63.
-        // This warp takes every kSplitWarps-th candidate of the transmitter,
-        // counted across depths.
-        int d = 1, c = 0, cnt = 0, global_c = 0;
+        __shared__ TileBounds all_bounds[kSplitWarps];
+        TileBounds& bounds = all_bounds[grp.index];
+        if (grp.rank == 0) {
+            const TileBounds tb = tile_bounds(Rf, active);
+            if (lane == 0) bounds = tb;
+        }
+        grp.sync();
+        __shared__ int all_c[kSplitWarps * kCandCap], all_d[kSplitWarps * kCandCap], all_n[kSplitWarps];
+        const int first = grp.index * grp.warps;
+        int* list_c = all_c + first * kCandCap;
+        int* list_d = all_d + first * kCandCap;
+        int* warp_n = all_n + first;
+        const int width = grp.warps * 32, cap = grp.warps * kCandCap;
+        const int tid = grp.rank * 32 + lane;
+        // Append the passing threads' (c, d) to the list, in thread order.
+        int listed = 0;
+        auto append = [&](bool pass, int c, int d) __attribute__((always_inline)) {
+            const unsigned mask = __ballot_sync(kFull, pass);
+            if (lane == 0) warp_n[grp.rank] = __popc(mask);
+            grp.sync();
+            int at = listed, total = 0;
+            for (int w = 0; w < grp.warps; ++w) {
+                if (w < grp.rank) at += warp_n[w];
+                total += warp_n[w];
+            }
+            if (pass) {
+                at += __popc(mask & lanemask_lt());
+                list_c[at] = c;
+                list_d[at] = d;
+            }
+            listed += total;
+            grp.sync();
+        };
+        int d = 0, c = 0, cnt = 0, first_g = 0;  // next candidate of the transmitter; candidates of lower depths
         long long base = 0;
         auto enter_depth = [&]() __attribute__((always_inline)) {
-            while (d <= p.max_depth) {
+            while (c >= cnt && d < p.max_depth) {
+                ++d;
+                first_g += cnt;
+                c = 0;
                 cnt = p.chain_count[t * kMaxDepth + (d - 1)];
                 base = p.chain_offset[t * kMaxDepth + (d - 1)];
-                c = (warp - global_c % kSplitWarps + kSplitWarps) % kSplitWarps;
-                global_c += cnt;
-                if (c < cnt) return;
-                ++d;
             }
         };
         enter_depth();
-        while (true) {
-            const bool cand_left = d <= p.max_depth;
-            int step;
-            if (qf >= 32) step = 3;
-            else if (qb >= 32) step = 2;
-            else if (qa >= 32) step = 1;
-            else if (cand_left) step = 0;
-            else if (qa > 0) step = 1;
-            else if (qb > 0) step = 2;
-            else if (qf > 0) step = 3;
-            else break;
-            if (step == 0) {
-                bool pass = active;
-                if (sizeof(T) == 4 && pass) pass = back_project_prefilter(sc, Rf, p.chain_pre + (base + c) * 2);
-                qa = queue_push(sh->qa, qa, pass, lane, c, d);
-                c += kSplitWarps;
-                if (c >= cnt) {
-                    ++d;
-                    enter_depth();
-                }
-            } else if (step == 1) {
-                process_a(qa < 32 ? qa : 32);
-            } else if (step == 2) {
-                process_b(qb < 32 ? qb : 32);
-            } else {
-                process_f(qf < 32 ? qf : 32);
+        bool last;
+        do {
+            // the next candidates that the tile may see, one test per thread
+            listed = 0;
+            while (c < cnt && listed <= cap - width) {
+                const int ct = c + tid;
+                append(ct < cnt && tile_may_reflect(p, bounds, base, ct, d), ct, d | (((first_g + ct) & 7) << 4));
+                c += width;
+                enter_depth();
             }
-        }
+            last = c >= cnt;
+            // drop those whose last leg one triangle blocks for the whole tile;
+            // the list is spread over the warps.  A warp with one or two
+            // candidates tests their legs directly.
+            const int n0 = listed;
+            if (n0 > 2 * grp.warps) listed = 0;
+            for (int b = listed; b < n0; b += width) {
+                const int per = (min(n0 - b, width) + grp.warps - 1) / grp.warps;
+                const int at = b + grp.rank * per + lane;
+                bool pass = lane < per && at < n0;
+                const int ec = pass ? list_c[at] : 0, ed = pass ? list_d[at] : 1;
+                if (pass) {
+                    ++rays;
+                    pass = !last_leg_blocked(p, bounds, p.chain_offset[t * kMaxDepth + ((ed & 15) - 1)], ec, stack);
+                }
+                append(pass, ec, ed);
+            }
+            // One loop drives the stages so each is inlined once.  Each pass
+            // runs one step, full batches first and the latest stage first: F,
+            // then B, then A, then the next candidate into queue A; partial
+            // batches only once nothing upstream can fill them.  A stage runs
+            // only while the queues it feeds hold fewer than 32 items, so no
+            // queue exceeds 63.  The group's warps take the candidates in turn;
+            // in FP64, whose warp sums are rounded to FP32 before they are
+            // added, warp w takes the candidates w (mod 8) of the whole table,
+            // so a cell's grouping does not depend on what its tile drops.
+            int e = sizeof(T) == 4 ? grp.rank : 0;
+            while (true) {
+                if (sizeof(T) == 8)
+                    while (e < listed && (list_d[e] >> 4) != grp.rank) ++e;
+                const bool cand_left = e < listed;
+                int step;
+                if (qf >= 32) step = 3;
+                else if (qb >= 32) step = 2;
+                else if (qa >= 32) step = 1;
+                else if (cand_left) step = 0;
+                else if (!last) break;
+                else if (qa > 0) step = 1;
+                else if (qb > 0) step = 2;
+                else if (qf > 0) step = 3;
+                else break;
+                if (step == 0) {
+                    const int ec = list_c[e], ed = list_d[e] & 15;
+                    bool pass = active;
+                    if (sizeof(T) == 4 && pass)
+                        pass = back_project_prefilter(sc, Rf, p.chain_pre + (p.chain_offset[t * kMaxDepth + (ed - 1)] + ec) * 2);
+                    qa = queue_push(sh->qa, qa, pass, lane, ec, ed);
+                    e += sizeof(T) == 4 ? grp.warps : 1;
+                } else if (step == 1) {
+                    process_a(qa < 32 ? qa : 32);
+                } else if (step == 2) {
+                    process_b(qb < 32 ? qb : 32);
+                } else {
+                    process_f(qf < 32 ? qf : 32);
+                }
+            }
+            grp.sync();
+        } while (!last);
         // fixed-order reduction of the warps' partial sums, one write per cell
         for (int f = 0; f < NF; ++f) {
             float* o = red + ((warp * 32 + lane) * NF + f) * 3;
@@ -532,13 +776,13 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
             o[1] = float(value_of(acc[f].im));
             o[2] = float(value_of(gain[f]));
         }
-        __syncthreads();
-        if (warp == 0 && active) {
+        grp.sync();
+        if (grp.rank == 0 && active) {
             const long long cell = (long long)t * p.num_rx + r;
             for (int f = 0; f < NF; ++f) {
                 Cx<T> sum = cx(T(0), T(0));
                 T g = T(0);
-                for (int w = 0; w < kSplitWarps; ++w) {
+                for (int w = warp; w < warp + grp.warps; ++w) {
                     const float* o = red + ((w * 32 + lane) * NF + f) * 3;
                     sum = sum + cx(T(o[0]), T(o[1]));
                     g = g + T(o[2]);
@@ -565,23 +809,82 @@ struct DiffShared {
 // runs at twice the occupancy of the field kernel and neither competes with
 // the other for instruction cache.
 
+// Does one triangle block every Q -> Rx segment between the edge and a tile?
+// The clamped stationary point moves along the edge with the receiver:
+// t* = ts + (tr - ts) rs / (rs + rr) is monotone in the receiver's edge
+// coordinate tr and, with the sign of tr - ts, in its edge distance rr, so its
+// range over the tile's bounds is spanned by the ends of their ranges.
+WCB_D bool edge_shaft_blocked(const SceneDev& sc, int edge, V3<double> S, const TileBounds& b, int* stack) {
+    const EdgeDev& ed = sc.edges[edge];
+    const V3<float> c = v3(float(ed.pos[0]), float(ed.pos[1]), float(ed.pos[2]));
+    const V3<float> e = v3(float(ed.dir[0]), float(ed.dir[1]), float(ed.dir[2]));
+    const float hl = float(ed.half_length);
+    const V3<float> ds = v3(float(S.x - ed.pos[0]), float(S.y - ed.pos[1]), float(S.z - ed.pos[2]));
+    const float ts = dot(ds, e);
+    const float rs = length(ds - e * ts);
+    const V3<float> mid = v3(0.5f * (b.lo[0] + b.hi[0]), 0.5f * (b.lo[1] + b.hi[1]), 0.5f * (b.lo[2] + b.hi[2]));
+    const V3<float> half = v3(0.5f * (b.hi[0] - b.lo[0]), 0.5f * (b.hi[1] - b.lo[1]), 0.5f * (b.hi[2] - b.lo[2]));
+    const V3<float> dm = mid - c;
+    const float tm = dot(dm, e);
+    const float rm = length(dm - e * tm);
+    const float tw = fabsf(e.x) * half.x + fabsf(e.y) * half.y + fabsf(e.z) * half.z;
+    const float rw = length(half);
+    const float size = fmaxf(norm1(mid) + norm1(half), norm1(c) + hl);
+    const float slack = 1e-3f + 2e-5f * (size + rs);
+    const float r_lo = fmaxf(rm - rw - slack, 0.f), r_hi = rm + rw + slack;
+    const float w_lo = rs / fmaxf(rs + r_hi, 1e-6f), w_hi = rs / fmaxf(rs + r_lo, 1e-6f);
+    const float d_lo = tm - tw - ts, d_hi = tm + tw - ts;
+    const float t_lo = ts + fminf(d_lo * w_lo, d_lo * w_hi) - slack, t_hi = ts + fmaxf(d_hi * w_lo, d_hi * w_hi) + slack;
+    const float q_lo = fminf(fmaxf(t_lo, -hl), hl), q_hi = fminf(fmaxf(t_hi, -hl), hl);
+    const V3<float> bias = v3(float(ed.bisector[0]), float(ed.bisector[1]), float(ed.bisector[2])) *
+                           float(kDiffractionRayBias);
+    Shaft s;
+    s.a[0] = c + e * q_lo + bias;
+    s.a[1] = c + e * q_hi + bias;
+    s.na = q_hi > q_lo ? 2 : 1;
+    for (int k = 0; k < 3; ++k) {
+        s.lo[k] = b.lo[k];
+        s.hi[k] = b.hi[k];
+    }
+    s.size = size;
+    s.side = 0.f;
+    Ignore ig = ignore_none();
+    ig.f0 = ed.face0;
+    ig.f1 = ed.face1;
+    return shaft_blocked(sc, (s.a[0] + s.a[1]) * 0.5f, mid, ig, s, stack);
+}
+
 // Visibility words of edges [j0, j0 + chunk) of each tile's transmitter: bit
 // `lane` of word (tile, j - j0) is set when both Tx -> Q and Q -> Rx are clear
 // for that lane's cell, Q the clamped stationary point on the edge moved by
 // kDiffractionRayBias along its exterior bisector.
+//
+// Issue bound (68-74 %).  One thread first tries to close a whole (tile, edge)
+// pair with one triangle (shaft.cuh), so a warp settles 32 pairs with one
+// divergent traversal where it took 32 coherent ones; only open pairs are
+// traced per cell, the receiver's leg first (49 % of the canyon's are clear,
+// against 88 % of the transmitter's).  It closes 77 % of the canyon's pairs and
+// 98.5 % of the 2048-box city's.  Before and after, on one B200: canyon 0.44 ->
+// 0.30-0.34 ms, four-transmitter batch 5.35 -> 3.1 ms, city 245 -> 60 ms.
 template <typename T>
-__global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, int stack_depth, int j0, int chunk,
+__global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, int tile_warps, int j0, int chunk,
                                                                  unsigned* vis_words) {
     extern __shared__ int smem[];
     int* stack = smem;
     const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const long long tile = blockIdx.x;
+    const TileGroup grp = tile_group(tile_warps);
+    const long long tile = grp.tile;
     int t = 0, r = 0;
     const bool active = tile_cell(p, tile, lane, &t, &r);
     const long long per_tx = tiles_per_tx(p);
     const int tw = int(tile / per_tx);
-    if (tw >= p.num_tx) return;
+    // one tile per warp: the block's eight tiles (a strip of neighbours) share a
+    // first test when they have the same transmitter, so a shaft that one
+    // triangle blocks for the whole strip costs one traversal instead of eight
+    const long long first_tile = (long long)blockIdx.x * kSplitWarps;
+    const bool strip = tile_warps == 1 && first_tile / per_tx == (first_tile + kSplitWarps - 1) / per_tx &&
+                       first_tile + kSplitWarps <= per_tx * p.num_tx;
+    if (tw >= p.num_tx) return;  // whole groups; never in a strip
     t = tw;
     const SceneDev& sc = p.sc;
     int* err = p.status;
@@ -594,55 +897,121 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
     const V3<float> Rf = active ? rx_point(p, r) : v3(0.f, 0.f, 0.f);
     const V3<double> R = cast3<double>(Rf);
     unsigned long long rays = 0;
-    for (int j = j0 + warp; j < jend; j += kSplitWarps) {
-        bool vis = false;
-        if (active) {
-            const EdgeDev& ed = sc.edges[list[j]];
-            const V3<double> c = v3(ed.pos[0], ed.pos[1], ed.pos[2]);
-            const V3<double> e = v3(ed.dir[0], ed.dir[1], ed.dir[2]);
-            const V3<double> ds = S - c;
-            const double ts = dot(ds, e);
-            const double rs = length(ds - e * ts);
-            const V3<double> dr = R - c;
-            const double tr = dot(dr, e);
-            const double rr = length(dr - e * tr);
-            const double t_star = (rs + rr) > 0.0 ? ts + (tr - ts) * rs / (rs + rr) : ts;
-            const double tc = fmin(fmax(t_star, -ed.half_length), ed.half_length);
-            const V3<double> qv_pt = c + e * tc + v3(ed.bisector[0], ed.bisector[1], ed.bisector[2]) * kDiffractionRayBias;
-            Ignore ig = ignore_none();
-            ig.f0 = ed.face0;
-            ig.f1 = ed.face1;
-            ++rays;
-            vis = !segment_blocked<T>(sc, ST, cast3<T>(qv_pt), ig, stack, err);
-            if (vis) {
+    __shared__ TileBounds all_bounds[kSplitWarps];
+    __shared__ int all_open[kSplitBlock], all_n[kSplitWarps];
+    TileBounds& bounds = all_bounds[grp.index];
+    int* open_edges = all_open + grp.index * grp.warps * 32;
+    int& num_open = all_n[grp.index];
+    if (grp.rank == 0) {
+        const TileBounds tb = tile_bounds(Rf, active);
+        if (lane == 0) bounds = tb;
+    }
+    const int width = grp.warps * 32;
+    __shared__ int strip_edges[kSplitBlock], strip_n;
+    const int span = strip ? kSplitBlock : width;
+    int m = 0, i0 = 0;
+    for (int jb = j0; jb < jend || i0 < m;) {
+        if (strip && i0 >= m) {
+            // the strip's next 256 edges
+            __syncthreads();
+            if (threadIdx.x == 0) strip_n = 0;
+            __syncthreads();
+            const int js = jb + threadIdx.x;
+            if (js < jend) {
+                TileBounds sb = all_bounds[0];
+                for (int w = 1; w < kSplitWarps; ++w)
+                    for (int k = 0; k < 3; ++k) {
+                        sb.lo[k] = fminf(sb.lo[k], all_bounds[w].lo[k]);
+                        sb.hi[k] = fmaxf(sb.hi[k], all_bounds[w].hi[k]);
+                    }
                 ++rays;
-                vis = !segment_blocked<T>(sc, cast3<T>(qv_pt), cast3<T>(R), ig, stack, err);
+                if (edge_shaft_blocked(sc, list[js], S, sb, stack)) {
+                    for (int w = 0; w < kSplitWarps; ++w) vis_words[(first_tile + w) * chunk + (js - j0)] = 0u;
+                } else {
+                    strip_edges[atomicAdd(&strip_n, 1)] = js;
+                }
             }
+            __syncthreads();
+            m = strip_n;
+            i0 = 0;
+            jb += span;
+            if (m == 0) continue;
+        } else if (!strip) {
+            m = min(span, jend - jb);
+            i0 = 0;
         }
-        const unsigned word = __ballot_sync(kFull, vis);
-        if (lane == 0) vis_words[tile * chunk + (j - j0)] = word;
+        if (grp.rank == 0 && lane == 0) num_open = 0;
+        grp.sync();
+        // one edge per thread: a pair whose Q -> tile shaft one triangle blocks
+        // has no visible cell
+        const int per = (min(m - i0, width) + grp.warps - 1) / grp.warps;
+        const int at = i0 + grp.rank * per + lane;
+        if (lane < per && at < m) {
+            const int jt = strip ? strip_edges[at] : jb + at;
+            ++rays;
+            const bool closed = edge_shaft_blocked(sc, list[jt], S, bounds, stack);
+            if (closed) vis_words[tile * chunk + (jt - j0)] = 0u;
+            else open_edges[atomicAdd(&num_open, 1)] = jt;
+        }
+        i0 += width;
+        if (!strip) jb += span;
+        grp.sync();
+        const int n = num_open;
+        for (int i = grp.rank; i < n; i += grp.warps) {
+            const int j = open_edges[i];
+            bool vis = false;
+            if (active) {
+                const EdgeDev& ed = sc.edges[list[j]];
+                const V3<double> c = v3(ed.pos[0], ed.pos[1], ed.pos[2]);
+                const V3<double> e = v3(ed.dir[0], ed.dir[1], ed.dir[2]);
+                const V3<double> ds = S - c;
+                const double ts = dot(ds, e);
+                const double rs = length(ds - e * ts);
+                const V3<double> dr = R - c;
+                const double tr = dot(dr, e);
+                const double rr = length(dr - e * tr);
+                const double t_star = (rs + rr) > 0.0 ? ts + (tr - ts) * rs / (rs + rr) : ts;
+                const double tc = fmin(fmax(t_star, -ed.half_length), ed.half_length);
+                const V3<double> qv_pt =
+                    c + e * tc + v3(ed.bisector[0], ed.bisector[1], ed.bisector[2]) * kDiffractionRayBias;
+                Ignore ig = ignore_none();
+                ig.f0 = ed.face0;
+                ig.f1 = ed.face1;
+                ++rays;
+                // the receiver's leg first: the edge list holds edges the Tx sees
+                vis = !segment_blocked<T>(sc, cast3<T>(qv_pt), cast3<T>(R), ig, stack, err);
+                if (vis) {
+                    ++rays;
+                    vis = !segment_blocked<T>(sc, ST, cast3<T>(qv_pt), ig, stack, err);
+                }
+            }
+            const unsigned word = __ballot_sync(kFull, vis);
+            if (lane == 0) vis_words[tile * chunk + (j - j0)] = word;
+        }
+        grp.sync();
     }
     if (p.ray_counter && p.freq_base == 0 && rays) atomicAdd(p.ray_counter, rays);
 }
 
 // UTD fields of the visible pairs of edges [j0, j0 + chunk).  The tile's
-// items are the set bits of its visibility words in (edge, lane) order; warp
-// w takes the contiguous w-th eighth of them, queues them and evaluates full
-// batches of 32, so the warps of a block finish together.  Per-cell sums are
+// items are the set bits of its visibility words in (edge, lane) order; each
+// warp of the tile's group takes a contiguous equal share of them, queues them
+// and evaluates full batches of 32, so the group's warps finish together.  Per-cell sums are
 // reduced over the warps in a fixed order.
 // With more than one chunk the running sums (9 values per cell and
 // frequency) pass between chunks through `carry`; the chunk that reaches the
 // end of the transmitter's edge list writes the outputs.  Chunk 0 always
 // runs, so a transmitter without visible edges still gets its zeros.
 template <typename T, int NF>
-__global__ void __launch_bounds__(kSplitBlock, 2) k_diffract_utd(MainParams p, int j0, int chunk,
+__global__ void __launch_bounds__(kSplitBlock, 2) k_diffract_utd(MainParams p, int tile_warps, int j0, int chunk,
                                                                  const unsigned* vis_words, T* carry) {
     extern __shared__ int smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     DiffShared<NF>* sh = reinterpret_cast<DiffShared<NF>*>(smem) + warp;
     float* red = reinterpret_cast<float*>(reinterpret_cast<DiffShared<NF>*>(smem) + kSplitWarps);
-    const long long tile = blockIdx.x;
+    const TileGroup grp = tile_group(tile_warps);
+    const long long tile = grp.tile;
     int t = 0, r = 0;
     const bool active = tile_cell(p, tile, lane, &t, &r);
     const long long per_tx = tiles_per_tx(p);
@@ -747,8 +1116,8 @@ __global__ void __launch_bounds__(kSplitBlock, 2) k_diffract_utd(MainParams p, i
         const int jj = b + lane;
         total += int(__reduce_add_sync(kFull, jj < nw ? unsigned(__popc(words[jj])) : 0u));
     }
-    const int lo = int((long long)total * warp / kSplitWarps);
-    const int hi = int((long long)total * (warp + 1) / kSplitWarps);
+    const int lo = int((long long)total * grp.rank / grp.warps);
+    const int hi = int((long long)total * (grp.rank + 1) / grp.warps);
     // skip, 32 words at a time, the words whose items all precede lo
     int jj = 0, seen = 0;
     for (; jj < nw; jj += 32) {
@@ -802,8 +1171,8 @@ __global__ void __launch_bounds__(kSplitBlock, 2) k_diffract_utd(MainParams p, i
             o[4 + 2 * k] = float(value_of(dv[f][k].im));
         }
     }
-    __syncthreads();
-    if (warp == 0 && active && (p.components & 4)) {
+    grp.sync();
+    if (grp.rank == 0 && active && (p.components & 4)) {
         const long long cell = (long long)t * p.num_rx + r;
         const long long cells = (long long)p.num_tx * p.num_rx;
         for (int f = 0; f < NF; ++f) {
@@ -816,7 +1185,7 @@ __global__ void __launch_bounds__(kSplitBlock, 2) k_diffract_utd(MainParams p, i
                 g = cr[2];
                 for (int k = 0; k < 3; ++k) v[k] = cx(cr[3 + 2 * k], cr[4 + 2 * k]);
             }
-            for (int w = 0; w < kSplitWarps; ++w) {
+            for (int w = warp; w < warp + grp.warps; ++w) {
                 const float* o = red + ((w * 32 + lane) * NF + f) * 9;
                 sum = sum + cx(T(o[0]), T(o[1]));
                 g = g + T(o[2]);

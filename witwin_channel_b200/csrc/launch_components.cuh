@@ -1,0 +1,104 @@
+// Definition of launch_components (launch.h); included by solve_f32.cu and
+// solve_f64.cu.
+#pragma once
+
+#include "internal.h"
+#include "kernels.cuh"
+#include "launch.h"
+
+namespace wcb {
+
+// Warps per 32-cell tile of the reflection and diffraction kernels.  One warp
+// per tile keeps its batches full and waits for nobody, but its tiles take
+// unequal times, so it needs many waves to even out; eight warps share a tile
+// when tiles are few.  Measured (one B200, sum of the two kernels' calls): the
+// 1024^2 large city (32,768 tiles) 93 ms at 1, 105 at 4, 123 at 8; four
+// transmitters on 128^2 and 320^2 (2,048 and 12,800 tiles) 27.7 ms at 1, 22.4
+// at 4, 25.6 at 8; a 90 x 70 town (216 tiles) 7.3 ms at 1, 4.5 at 8.  FP64
+// keeps eight: its warps' sums are rounded to FP32 before they are added, so
+// another grouping would be another result.
+template <typename T>
+static int tile_warps_for(long long tiles) {
+    if (sizeof(T) == 8) return 8;
+    return tiles >= 16384 ? 1 : tiles >= 1024 ? 4 : 8;
+}
+
+// LoS+transmission and diffraction go on `stream`, reflection on `side` (its
+// candidate tables were built there); the caller joins the streams before
+// the finalize kernel.
+template <typename T, int NF>
+static void launch_nf(const MainParams& q0, unsigned blocks, int sdepth, size_t stack_bytes, cudaStream_t stream,
+               cudaStream_t side, ComponentEvents* evs, const DiffractionPlan& dp) {
+    const long long tiles = tiles_per_tx(q0) * q0.num_tx;
+    const int tw = tile_warps_for<T>(tiles);
+    const unsigned grid = unsigned((tiles * tw + kSplitWarps - 1) / kSplitWarps);
+    const size_t split_stack = size_t(sdepth) * kSplitBlock * 4;
+    const int c = q0.components;
+    MainParams q = q0;
+    unsigned long long* rc = q0.ray_counter;
+    if (c & 2) {
+        if (evs) cudaEventRecord(evs->start[1], side);
+        q.ray_counter = rc ? rc + 1 : nullptr;
+        const size_t bytes = split_stack + kSplitWarps * sizeof(ReflShared<NF>) + size_t(kSplitWarps) * 32 * NF * 3 * 4;
+        static bool attr = false;
+        if (!attr) {
+            cudaFuncSetAttribute(k_reflect<T, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            attr = true;
+        }
+        k_reflect<T, NF><<<grid, kSplitBlock, bytes, side>>>(q, sdepth, tw);
+        note_launch();
+        if (evs) cudaEventRecord(evs->end[1], side);
+    }
+    if (evs) cudaEventRecord(evs->start[0], stream);
+    if (c & (1 | 8)) {
+        q.ray_counter = rc ? rc + 0 : nullptr;
+        k_los_trans<T, NF><<<blocks, kCompBlock, stack_bytes, stream>>>(q);
+        note_launch();
+    }
+    if (evs) cudaEventRecord(evs->end[0], stream);
+    if (evs) cudaEventRecord(evs->start[2], stream);
+    if ((c & 4) && dp.chunks > 0) {
+        q.ray_counter = rc ? rc + 2 : nullptr;
+        const size_t bytes = kSplitWarps * sizeof(DiffShared<NF>) + size_t(kSplitWarps) * 32 * NF * 9 * 4;
+        static bool attr = false;
+        if (!attr) {
+            cudaFuncSetAttribute(k_diffract_vis<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            cudaFuncSetAttribute(k_diffract_utd<T, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            attr = true;
+        }
+        for (int k = 0; k < dp.chunks; ++k) {
+            const int j0 = k * dp.chunk;
+            if (dp.run_vis) {
+                std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
+                if (evs) {
+                    cudaEventCreate(&ev.first);
+                    cudaEventCreate(&ev.second);
+                    cudaEventRecord(ev.first, stream);
+                }
+                k_diffract_vis<T><<<grid, kSplitBlock, split_stack, stream>>>(q, tw, j0, dp.chunk, dp.words);
+                note_launch();
+                if (evs) {
+                    cudaEventRecord(ev.second, stream);
+                    evs->vis.push_back(ev);
+                }
+            }
+            k_diffract_utd<T, NF><<<grid, kSplitBlock, bytes, stream>>>(q, tw, j0, dp.chunk, dp.words,
+                                                                           static_cast<T*>(dp.carry));
+            note_launch();
+        }
+    }
+    if (evs) cudaEventRecord(evs->end[2], stream);
+}
+
+template <typename T>
+void launch_components(const MainParams& q, int nf, unsigned blocks, int sdepth, size_t stack_bytes, cudaStream_t stream,
+                       cudaStream_t side, ComponentEvents* evs, const DiffractionPlan& dp) {
+    switch (nf) {
+        case 1: launch_nf<T, 1>(q, blocks, sdepth, stack_bytes, stream, side, evs, dp); break;
+        case 2: launch_nf<T, 2>(q, blocks, sdepth, stack_bytes, stream, side, evs, dp); break;
+        case 3: launch_nf<T, 3>(q, blocks, sdepth, stack_bytes, stream, side, evs, dp); break;
+        default: launch_nf<T, 4>(q, blocks, sdepth, stack_bytes, stream, side, evs, dp); break;
+    }
+}
+
+}  // namespace wcb

@@ -29,6 +29,7 @@
 #include "solve.h"
 #include "utd.cuh"
 #include "kernels.cuh"
+#include "launch.h"
 
 namespace wcb {
 
@@ -357,14 +358,6 @@ __global__ void k_compact_flags(int n, const int* flags, int* list, int* count) 
 // ------------------------------------------------------------ main kernel
 
 
-// Start/end events of the four per-cell kernels (LoS+transmission,
-// reflection, diffraction, finalize), each recorded on the kernel's stream.
-struct ComponentEvents {
-    cudaEvent_t start[4] = {nullptr, nullptr, nullptr, nullptr};
-    cudaEvent_t end[4] = {nullptr, nullptr, nullptr, nullptr};
-    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> vis;  // around each diffraction visibility launch
-};
-
 // Diffraction edge chunking: the visibility words of one chunk take at most
 // kVisWordBudget 32-bit words (64 MiB), one word per (tile, edge).  The
 // environment variable WCB_DIFFRACTION_CHUNK_WORDS lowers the budget (tests
@@ -380,14 +373,6 @@ static long long vis_word_budget() {
     return kVisWordBudget;
 }
 
-struct DiffractionPlan {
-    int chunk = 0;           // edges per chunk
-    int chunks = 0;          // chunks covering the scene's edge count
-    unsigned* words = nullptr;
-    void* carry = nullptr;   // running per-cell sums between chunks (chunks > 1)
-    bool run_vis = true;     // false when this frequency block reuses the words
-};
-
 static long long host_tiles_per_tx(const wcb_solve_desc& d) {
     if (d.rx_kind == 1) return (long long)((d.grid_rows + 7) / 8) * ((d.grid_cols + 3) / 4);
     return (d.num_rx + 31) / 32;
@@ -402,82 +387,6 @@ static DiffractionPlan diffraction_plan(const SceneDev& sc, const wcb_solve_desc
     dp.chunk = int(chunk);
     dp.chunks = int((sc.num_edges + chunk - 1) / chunk);
     return dp;
-}
-
-// LoS+transmission and diffraction go on `stream`, reflection on `side` (its
-// candidate tables were built there); the caller joins the streams before
-// the finalize kernel.
-template <typename T, int NF>
-void launch_nf(const MainParams& q0, unsigned blocks, int sdepth, size_t stack_bytes, cudaStream_t stream,
-               cudaStream_t side, ComponentEvents* evs, const DiffractionPlan& dp) {
-    const unsigned tiles = unsigned(tiles_per_tx(q0) * q0.num_tx);
-    const size_t split_stack = size_t(sdepth) * kSplitBlock * 4;
-    const int c = q0.components;
-    MainParams q = q0;
-    unsigned long long* rc = q0.ray_counter;
-    if (c & 2) {
-        if (evs) cudaEventRecord(evs->start[1], side);
-        q.ray_counter = rc ? rc + 1 : nullptr;
-        const size_t bytes = split_stack + kSplitWarps * sizeof(ReflShared<NF>) + size_t(kSplitWarps) * 32 * NF * 3 * 4;
-        static bool attr = false;
-        if (!attr) {
-            cudaFuncSetAttribute(k_reflect<T, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            attr = true;
-        }
-        k_reflect<T, NF><<<tiles, kSplitBlock, bytes, side>>>(q, sdepth);
-        note_launch();
-        if (evs) cudaEventRecord(evs->end[1], side);
-    }
-    if (evs) cudaEventRecord(evs->start[0], stream);
-    if (c & (1 | 8)) {
-        q.ray_counter = rc ? rc + 0 : nullptr;
-        k_los_trans<T, NF><<<blocks, kCompBlock, stack_bytes, stream>>>(q);
-        note_launch();
-    }
-    if (evs) cudaEventRecord(evs->end[0], stream);
-    if (evs) cudaEventRecord(evs->start[2], stream);
-    if ((c & 4) && dp.chunks > 0) {
-        q.ray_counter = rc ? rc + 2 : nullptr;
-        const size_t bytes = kSplitWarps * sizeof(DiffShared<NF>) + size_t(kSplitWarps) * 32 * NF * 9 * 4;
-        static bool attr = false;
-        if (!attr) {
-            cudaFuncSetAttribute(k_diffract_vis<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            cudaFuncSetAttribute(k_diffract_utd<T, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            attr = true;
-        }
-        for (int k = 0; k < dp.chunks; ++k) {
-            const int j0 = k * dp.chunk;
-            if (dp.run_vis) {
-                std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
-                if (evs) {
-                    cudaEventCreate(&ev.first);
-                    cudaEventCreate(&ev.second);
-                    cudaEventRecord(ev.first, stream);
-                }
-                k_diffract_vis<T><<<tiles, kSplitBlock, split_stack, stream>>>(q, sdepth, j0, dp.chunk, dp.words);
-                note_launch();
-                if (evs) {
-                    cudaEventRecord(ev.second, stream);
-                    evs->vis.push_back(ev);
-                }
-            }
-            k_diffract_utd<T, NF><<<tiles, kSplitBlock, bytes, stream>>>(q, j0, dp.chunk, dp.words,
-                                                                        static_cast<T*>(dp.carry));
-            note_launch();
-        }
-    }
-    if (evs) cudaEventRecord(evs->end[2], stream);
-}
-
-template <typename T>
-void launch_components(const MainParams& q, int nf, unsigned blocks, int sdepth, size_t stack_bytes, cudaStream_t stream,
-                       cudaStream_t side, ComponentEvents* evs, const DiffractionPlan& dp) {
-    switch (nf) {
-        case 1: launch_nf<T, 1>(q, blocks, sdepth, stack_bytes, stream, side, evs, dp); break;
-        case 2: launch_nf<T, 2>(q, blocks, sdepth, stack_bytes, stream, side, evs, dp); break;
-        case 3: launch_nf<T, 3>(q, blocks, sdepth, stack_bytes, stream, side, evs, dp); break;
-        default: launch_nf<T, 4>(q, blocks, sdepth, stack_bytes, stream, side, evs, dp); break;
-    }
 }
 
 // One non-blocking side stream per device, created on first use.
