@@ -7,11 +7,10 @@
 //   coefficient: one FP64 forward sweep that keeps its intermediates, then one
 //   reverse sweep that returns the gradient of a real loss with respect to
 //   every input at once (Tx and Rx positions, the edge frame, the frequency,
-//   and eps_r / sigma of both face materials).  The two subfunctions with many
-//   internal branches -- a mended KP term (five inputs) and a half-space
-//   Fresnel face factor (four inputs) -- give their local Jacobians through
-//   dual lanes inside the forward sweep; everything else is differentiated by
-//   hand.  Each branch (floors, clamps, the wedge-angle wrap, the corner
+//   and eps_r / sigma of both face materials).  A mended KP term (five inputs)
+//   and a half-space face factor (four inputs) form their local Jacobians in
+//   closed form inside the forward sweep (as dual lanes they cost the kernel
+//   most of its time).  Each branch (floors, clamps, the wedge-angle wrap, the corner
 //   selection) is differentiated on the side the forward value took, the same
 //   rule the dual-number evaluation follows, so both give the same
 //   derivatives up to rounding.
@@ -45,23 +44,166 @@ WCB_HD Cx<Dual<N>> phasor_kd(const Dual<N>& k, const Dual<N>& d) {
     return phasor_neg_kd(k, d);
 }
 
-// |(1+j)/2 - (C(x) + jS(x))| with d/dx (C + jS) = exp(j pi x^2 / 2).
+// |(1+j)/2 - (C(x) + jS(x))| and its derivative, d/dx (C + jS) = exp(j pi x^2 / 2).
+WCB_HD double fresnel_complement_abs_grad(double x, double* grad) {
+    const double ax = fabs(x);
+    const Cx<double> e = fresnel_phasor<double>(ax);
+    Cx<double> c = fresnel_pos<double>(ax).complement(ax, e);
+    if (x < 0.0) c = cx(1.0, 1.0) - c;
+    const double a = cabs(c);
+    *grad = a > 0.0 ? -(c.re * e.re + c.im * e.im) / a : 0.0;
+    return a;
+}
 template <int N>
 WCB_HD Dual<N> fresnel_complement_abs(const Dual<N>& x) {
-    const double xv = x.v;
-    Cx<double> c;
-    if (xv >= 0.0) {
-        c = fresnel_pos<double>(xv, true).complement;
-    } else {
-        c = cx(1.0, 1.0) - fresnel_pos<double>(-xv, true).complement;
-    }
-    const double a = hypot(c.re, c.im);
-    double ph = kPi / 2 * xv * xv;
-    ph = ph - kTwoPi * floor(ph / kTwoPi);
-    double es, ec;
-    sincos(ph, &es, &ec);
-    const double g = a > 0.0 ? -(c.re * ec + c.im * es) / a : 0.0;
+    double g;
+    const double a = fresnel_complement_abs_grad(x.v, &g);
     return chain(a, g, x);
+}
+
+// One KP term (kp_term) with its derivatives by beta, n and kl:
+// v = cot(eps/(2n)) F(X), X = 2 kl sin^2(eps/2), eps = pi + s beta - 2 pi n m with the
+// integer m constant, F' = F (1/(2X) + j) - j.
+struct KpJet {
+    Cx<double> v, db, dn, dkl;
+};
+inline WCB_HD_OOL KpJet kp_jet(double beta, double n, double kl, int s) {
+    const double two_n_pi = 2.0 * n * kPi;
+    const double arg = kPi + s * beta;
+    const double m = s_round(arg / two_n_pi);
+    const double eps = arg - two_n_pi * m;
+    KpJet j;
+    Cx<double> de;
+    if (fabs(eps) < 1e-9) {
+        // v = n ej (sg sqrt(2 pi kl) - 2 ej kl eps), ej^2 = j
+        const double is2 = 0.70710678118654752440, sg = eps < 0 ? -1.0 : 1.0;
+        const double r = s_sqrt(kTwoPi * kl);
+        const Cx<double> lead = cx(is2 * sg, is2 * sg);
+        const Cx<double> per_n = lead * r - cx(0.0, 2.0 * kl * eps);
+        j.v = per_n * n;
+        j.dn = per_n;
+        de = cx(0.0, -2.0 * kl * n);
+        j.dkl = lead * (n * (r > 0.0 ? 0.5 * kTwoPi / r : 0.0)) - cx(0.0, 2.0 * eps * n);
+    } else {
+        const double inv2n = 0.5 / n;
+        double sh, ch, se, ce;
+        s_sincos(eps * inv2n, &sh, &ch);
+        s_sincos(0.5 * eps, &se, &ce);
+        const double inv_sh = 1.0 / sh;
+        const double cot = ch * inv_sh;
+        const double X = 2.0 * kl * se * se;
+        const Cx<double> F = transition<double>(X);
+        Cx<double> dF = cx(0.0, 0.0);
+        if (X > 0.0) {
+            const double i2x = 0.5 / X;
+            dF = cx(F.re * i2x - F.im, F.im * i2x + F.re - 1.0);
+        }
+        const Cx<double> cdF = dF * cot;
+        const Cx<double> q = F * (inv_sh * inv_sh * inv2n);  // F / (2 n sin^2)
+        j.v = F * cot;
+        de = cdF * (2.0 * kl * se * ce) - q;
+        j.dn = q * (eps / n);
+        j.dkl = cdF * (2.0 * se * se);
+    }
+    j.db = de * double(s);
+    j.dn = j.dn - de * (kTwoPi * m);
+    return j;
+}
+
+// A mended KP term (mended_term) with its derivatives by beta, n, kl, t_mono
+// and gamma.
+struct MendedJet {
+    Cx<double> v, db, dn, dkl, dt, dg;
+};
+WCB_HD MendedJet mended_jet(double beta, double nn, double kl, double t_mono, double gamma, int sgn,
+                            bool incident_group) {
+    double b_star, db_star = 0.0;  // the corner and its derivative by n
+    if (incident_group) {
+        b_star = fabs(beta - kPi) <= fabs(beta + kPi) ? kPi : -kPi;
+    } else {
+        const double other = (2.0 * nn - 1.0) * kPi;
+        if (fabs(beta - kPi) <= fabs(beta - other)) {
+            b_star = kPi;
+        } else {
+            b_star = other;
+            db_star = kTwoPi;
+        }
+    }
+    const double delta = beta - b_star;
+    // the windows exp(-(delta / (c sqrt(2 pi / kl)))^2) = exp(-rate kl delta^2)
+    constexpr double rate_w = 1.0 / (16.0 * kTwoPi), rate_b = 1.0 / (kCBlend * kCBlend * kTwoPi);
+    double w = s_exp(-rate_w * kl * delta * delta);
+    if (w <= kWindowCutoff) w = 0.0;
+    KpJet a = kp_jet(beta, nn, kl, sgn);
+    MendedJet r;
+    if (w == 0.0) {
+        // no odd part: v t_mono
+        r.v = a.v * t_mono;
+        r.db = a.db * t_mono;
+        r.dn = a.dn * t_mono;
+        r.dkl = a.dkl * t_mono;
+        r.dt = a.v;
+        r.dg = cx(0.0, 0.0);
+        return r;
+    }
+    const KpJet b = kp_jet(2.0 * b_star - beta, nn, kl, sgn);
+    const double wb = s_exp(-rate_b * kl * delta * delta);
+    const double blend = wb + (1.0 - wb) * t_mono;
+    const Cx<double> half = (a.v - b.v) * 0.5;
+    const Cx<double> odd = half * w;
+    const double gb = gamma * blend;
+    // x stands for beta, n, kl: d odd = (da - db) w / 2 + half dw
+    const double wd = -2.0 * rate_w * kl * delta * w, bd = -2.0 * rate_b * kl * delta * wb * (1.0 - t_mono) * gamma;
+    const double wk = -rate_w * delta * delta * w, bk = -rate_b * delta * delta * wb * (1.0 - t_mono) * gamma;
+    const Cx<double> mirror_n = b.dn + b.db * (2.0 * db_star);
+    const Cx<double> ob = (a.db + b.db) * (0.5 * w) + half * wd;
+    const Cx<double> on = (a.dn - mirror_n) * (0.5 * w) - half * (wd * db_star);
+    const Cx<double> ok = (a.dkl - b.dkl) * (0.5 * w) + half * wk;
+    r.v = (a.v - odd) * t_mono + odd * gb;
+    r.db = (a.db - ob) * t_mono + ob * gb + odd * bd;
+    r.dn = (a.dn - on) * t_mono + on * gb - odd * (bd * db_star);
+    r.dkl = (a.dkl - ok) * t_mono + ok * gb + odd * bk;
+    r.dt = a.v - odd + odd * (gamma * (1.0 - wb));
+    r.dg = odd * blend;
+    return r;
+}
+
+// Half-space face factors (halfspace_fresnel) at the wedge angle `angle` with
+// their derivatives by angle, eps_r, sigma_e and frequency.
+struct FaceJet {
+    Cx<double> te, tm, dte[4], dtm[4];
+};
+WCB_HD void face_jet(double angle, const Slab<double>& m, double f, FaceJet& out) {
+    double sn, cs;
+    s_sincos(angle, &sn, &cs);
+    const double omega = s_max(kTwoPi * f, kUtdSmallEps);
+    const double raw = fabs(sn);
+    const bool ct_in = raw >= kUtdSmallEps && raw <= 1.0;
+    const double ct = fmin(fmax(raw, kUtdSmallEps), 1.0);
+    const double dct = ct_in ? (sn < 0.0 ? -cs : cs) : 0.0;  // by the angle
+    const bool eps_in = m.eps_r >= kUtdSmallEps, sig_in = m.sigma_e >= 0.0;
+    const double loss = (sig_in ? m.sigma_e : 0.0) / (omega * kEps0);
+    const Cx<double> eta = cx(eps_in ? m.eps_r : kUtdSmallEps, -loss);
+    const double mu = fmax(m.mu_r, kUtdSmallEps);
+    const double sin2 = fmax(1.0 - ct * ct, 0.0);
+    const Cx<double> root = csqrt(eta * mu - cx(sin2, 0.0));
+    const Cx<double> one = cx(1.0, 0.0);
+    const Cx<double> inv_root = one / root;
+    const Cx<double> a = cx(mu * ct, 0.0), b = eta * ct;
+    const Cx<double> ia = one / (a + root), ib = one / (b + root);
+    out.te = (a - root) * ia * m.gain;
+    out.tm = (b - root) * ib * m.gain;
+    // d((x - s)/(x + s)) = 2 (s dx - x ds) / (x + s)^2
+    const Cx<double> qa = ia * ia * (2.0 * m.gain), qb = ib * ib * (2.0 * m.gain);
+    auto lane = [&](int l, double dc, Cx<double> deta) {
+        const Cx<double> ds = (deta * mu + cx(2.0 * ct * dc, 0.0)) * inv_root * 0.5;
+        out.dte[l] = (root * (mu * dc) - a * ds) * qa;
+        out.dtm[l] = (root * (deta * ct + eta * dc) - b * ds) * qb;
+    };
+    lane(0, dct, cx(0.0, 0.0));
+    lane(1, 0.0, cx(eps_in ? 1.0 : 0.0, 0.0));
+    lane(2, 0.0, cx(0.0, sig_in ? -1.0 / (omega * kEps0) : 0.0));
+    lane(3, 0.0, cx(0.0, kTwoPi * f >= kUtdSmallEps ? loss * kTwoPi / omega : 0.0));
 }
 
 // ---------------------------------------------------------------- edge frame
@@ -212,18 +354,20 @@ WCB_HD Cx<double> utd_record_vjp(const UtdRecordIn& in, double sq, double gg, do
     const double sigma = sqrt(k * kappa / kPi);
     const double a_hi = sigma * (hl - t_star);
     const double a_lo = -(sigma * (-hl - t_star));
-    double hi_abs, lo_abs, dhi, dlo;
+    double hi_abs = 0.0, lo_abs = 0.0, dhi = 0.0, dlo = 0.0;
     {
-        Dual<1> x(a_hi);
-        x.d[0] = 1.0;
-        const Dual<1> r = fresnel_complement_abs(x);
-        hi_abs = r.v;
-        dhi = r.d[0];
-        x = Dual<1>(a_lo);
-        x.d[0] = 1.0;
-        const Dual<1> r2 = fresnel_complement_abs(x);
-        lo_abs = r2.v;
-        dlo = r2.d[0];
+#pragma unroll 1
+        for (int end = 0; end < 2; ++end) {
+            double g1;
+            const double v = fresnel_complement_abs_grad(end == 0 ? a_hi : a_lo, &g1);
+            if (end == 0) {
+                hi_abs = v;
+                dhi = g1;
+            } else {
+                lo_abs = v;
+                dlo = g1;
+            }
+        }
     }
     const double tm_raw = 1.0 - kIs2 * lo_abs - kIs2 * hi_abs;
     const bool tm_in = tm_raw >= 0.0 && tm_raw <= 1.0;
@@ -234,40 +378,24 @@ WCB_HD Cx<double> utd_record_vjp(const UtdRecordIn& in, double sq, double gg, do
     const bool ex_in = ex_raw <= 80.0;
     const double E = s_exp(ex_in ? ex_raw : 80.0);
     const double gamma = 1.0 / (1.0 + E);
-    // face factors with their Jacobians (lanes: angle, eps_r, sigma_e, frequency)
-    Cx<double> r_te[2] = {cx(0.0, 0.0), cx(0.0, 0.0)}, r_tm[2] = {cx(0.0, 0.0), cx(0.0, 0.0)};
-    Cx<double> dte[2][4], dtm[2][4];
+    // face factors with their Jacobians (angle, eps_r, sigma_e, frequency)
+    FaceJet fj[2];
+    fj[1].te = fj[1].tm = cx(0.0, 0.0);
     const int faces = fr.face_n ? 2 : 1;
 #pragma unroll 1
-    for (int face = 0; face < faces; ++face) {
-        const Slab<double>& m = face == 0 ? in.m0 : in.mn;
-        Dual<4> ang(face == 0 ? phi_p : npi - phi), er(m.eps_r), sg(m.sigma_e), fq(in.f);
-        for (int l = 0; l < 4; ++l) ang.d[l] = er.d[l] = sg.d[l] = fq.d[l] = 0.0;
-        ang.d[0] = er.d[1] = sg.d[2] = fq.d[3] = 1.0;
-        const Slab<Dual<4>> md{er, sg, Dual<4>(m.mu_r), Dual<4>(m.gain), Dual<4>(m.thickness)};
-        Cx<Dual<4>> te, tm;
-        halfspace_fresnel(s_sin(ang), md, fq, &te, &tm);
-        r_te[face] = cx(te.re.v, te.im.v);
-        r_tm[face] = cx(tm.re.v, tm.im.v);
-        for (int l = 0; l < 4; ++l) {
-            dte[face][l] = cx(te.re.d[l], te.im.d[l]);
-            dtm[face][l] = cx(tm.re.d[l], tm.im.d[l]);
-        }
-    }
+    for (int face = 0; face < faces; ++face)
+        face_jet(face == 0 ? phi_p : npi - phi, face == 0 ? in.m0 : in.mn, in.f, fj[face]);
     const double bm = phi - phi_p, bp = phi + phi_p;
-    // the four mended KP terms with their Jacobians (lanes: beta, n, kl, t_mono, gamma)
-    Cx<double> T[4], dT[4][5];
+    // the four mended KP terms with their Jacobians (beta, n, kl, t_mono, gamma)
+    Cx<double> T[4];
+    MendedJet mj[4];
 #pragma unroll 1
     for (int qq = 0; qq < 4; ++qq) {
         const bool incident = qq < 2;
-        Dual<5> b(incident ? bm : bp), n5(nn), k5(kl), tm5(t_mono), g5(gamma);
-        for (int l = 0; l < 5; ++l) b.d[l] = n5.d[l] = k5.d[l] = tm5.d[l] = g5.d[l] = 0.0;
-        b.d[0] = n5.d[1] = k5.d[2] = tm5.d[3] = g5.d[4] = 1.0;
-        const Cx<Dual<5>> r = mended_term(b, n5, k5, tm5, g5, (qq & 1) ? -1 : +1, incident);
-        T[qq] = cx(r.re.v, r.im.v);
-        for (int l = 0; l < 5; ++l) dT[qq][l] = cx(r.re.d[l], r.im.d[l]);
+        mj[qq] = mended_jet(incident ? bm : bp, nn, kl, t_mono, gamma, (qq & 1) ? -1 : +1, incident);
     }
-    const Cx<double> rn_te = r_te[1], rn_tm = r_tm[1], r0_te = r_te[0], r0_tm = r_tm[0];
+    for (int qq = 0; qq < 4; ++qq) T[qq] = mj[qq].v;
+    const Cx<double> rn_te = fj[1].te, rn_tm = fj[1].tm, r0_te = fj[0].te, r0_tm = fj[0].tm;
     const Cx<double> sum_soft = T[0] + T[1] + rn_te * T[2] + r0_te * T[3];
     const Cx<double> sum_hard = T[0] + T[1] + rn_tm * T[2] + r0_tm * T[3];
     const double pre_mag = 1.0 / (2.0 * nn * sqrt(kTwoPi * k) * sin_b);
@@ -379,19 +507,19 @@ WCB_HD Cx<double> utd_record_vjp(const UtdRecordIn& in, double sq, double gg, do
     rtmb[0] = shb_ * cconj(T[3]);
     double bmb = 0.0, bpb = 0.0, klb = 0.0, t_monob = 0.0, gammab = 0.0;
     for (int qq = 0; qq < 4; ++qq) {
-        const double cbeta = rdot(Tb[qq], dT[qq][0]);
+        const double cbeta = rdot(Tb[qq], mj[qq].db);
         if (qq < 2) bmb += cbeta;
         else bpb += cbeta;
-        nb += rdot(Tb[qq], dT[qq][1]);
-        klb += rdot(Tb[qq], dT[qq][2]);
-        t_monob += rdot(Tb[qq], dT[qq][3]);
-        gammab += rdot(Tb[qq], dT[qq][4]);
+        nb += rdot(Tb[qq], mj[qq].dn);
+        klb += rdot(Tb[qq], mj[qq].dkl);
+        t_monob += rdot(Tb[qq], mj[qq].dt);
+        gammab += rdot(Tb[qq], mj[qq].dg);
     }
     double phib = bmb + bpb, phi_pb = bpb - bmb;
     // face factors
     for (int face = 0; face < faces; ++face) {
         double lane[4];
-        for (int l = 0; l < 4; ++l) lane[l] = rdot(rteb[face], dte[face][l]) + rdot(rtmb[face], dtm[face][l]);
+        for (int l = 0; l < 4; ++l) lane[l] = rdot(rteb[face], fj[face].dte[l]) + rdot(rtmb[face], fj[face].dtm[l]);
         if (face == 0) {
             phi_pb += lane[0];
             g.eps0 += lane[1];
