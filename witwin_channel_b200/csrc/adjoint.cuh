@@ -12,6 +12,7 @@
 #include "paths.cuh"
 #include "solve.h"
 #include "utd.cuh"
+#include "reflection_adjoint.cuh"
 #include "utd_adjoint.cuh"
 
 namespace wcb {
@@ -573,6 +574,104 @@ __global__ void __launch_bounds__(kBlock) k_vjp_diffraction(AdjParams p) {
     if (ps.mn >= 0) {
         put(p.base_meps + ps.mn, g.epsn);
         put(p.base_msig + ps.mn, g.sign);
+    }
+}
+
+// Reverse mode over the reflection records: one thread per record, the pairs
+// in the same order as the diffraction kernel's.
+static __global__ void __launch_bounds__(kBlock) k_vjp_reflection(AdjParams p) {
+    const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (j >= p.order_count) return;
+    const long long i = p.order[p.order_begin + j];
+    const RowRec row = p.rows[p.selected[i]];
+    if (row.component != 1 || row.depth < 1) return;
+    const int d = min(int(row.depth), kMaxDepth);
+    const int t = row.tx, r = row.rx;
+    auto vtx = [&](int v) {
+        const float* x = p.sc.vertices + 3 * v;
+        return v3(double(x[0]), double(x[1]), double(x[2]));
+    };
+    ReflectionRecordIn<kMaxDepth> in;
+    in.depth = d;
+    in.S = v3(double(p.tx_pos[3 * t]), double(p.tx_pos[3 * t + 1]), double(p.tx_pos[3 * t + 2]));
+    const V3<Dual<0>> rq = receiver(p, Plain<0>{}, r);
+    in.R = v3(rq.x.v, rq.y.v, rq.z.v);
+    in.tx_pol = v3(double(p.tx_pol[3 * t]), double(p.tx_pol[3 * t + 1]), double(p.tx_pol[3 * t + 2]));
+    const float* rp = p.rx_pol + (long long)r * p.rx_pol_stride;
+    in.rx_pol = v3(double(rp[0]), double(rp[1]), double(rp[2]));
+    in.f = p.freq;
+    for (int q = 0; q < d; ++q) {
+        const int* f = p.sc.faces + 3 * row.seq[q];
+        const V3<double> a = vtx(f[0]);
+        in.n[q] = unit_face_normal(a, vtx(f[1]), vtx(f[2]));
+        in.off[q] = dot(in.n[q], a);
+        const int m = p.sc.face_material[row.seq[q]];
+        in.slab[q] = Slab<double>{double(p.eps_r[m]), double(p.sigma_e[m]), double(p.mu_r[m]), double(p.gain[m]),
+                                  double(p.thickness[m])};
+    }
+    const double sq = sqrt(fmax(double(p.tx_power[t]), 0.0));
+    ReflectionRecordGrad<kMaxDepth> g;
+    const Cx<double> pf = reflection_record_vjp(in, sq, p.g_gain ? p.g_gain[i] : 0.0, p.g_re ? p.g_re[i] : 0.0,
+                                                p.g_im ? p.g_im[i] : 0.0, g);
+    if (p.row_field) {
+        p.row_field[2 * i] = pf.re;
+        p.row_field[2 * i + 1] = pf.im;
+    }
+    long long o = p.offsets[i];
+    const long long o_end = o + p.counts[i];
+    auto put = [&](int id, double c) {
+        if (o >= o_end) return;  // never past the record's counted slots
+        if (!isfinite(c)) c = 0.0;
+        p.out_ids[o] = unsigned(id);
+        p.out_vals[o] = c;
+        ++o;
+    };
+    auto put3 = [&](int id, V3<double> c) {
+        put(id, c.x);
+        put(id + 1, c.y);
+        put(id + 2, c.z);
+    };
+    if (p.want & kWantTx) put3(p.base_tx + 3 * t, g.S);
+    if ((p.want & kWantRx) && p.rx_kind == 0) put3(p.base_rx + 3 * r, g.R);
+    if (p.want & kWantFreq) put(p.gid_freq, g.f);
+    if (p.want & kWantVertices) {
+        // the planes' gradients to their faces' vertices; a vertex of several
+        // faces is written once, at its first use, with the sum
+        V3<double> fg[kMaxDepth][3];
+        for (int q = 0; q < d; ++q) {
+            const int* f = p.sc.faces + 3 * row.seq[q];
+            const V3<double> a = vtx(f[0]);
+            for (int c = 0; c < 3; ++c) fg[q][c] = v3(0.0, 0.0, 0.0);
+            face_normal_vjp(a, vtx(f[1]), vtx(f[2]), g.n[q] + a * g.off[q], fg[q][0], fg[q][1], fg[q][2]);
+            fg[q][0] = fg[q][0] + in.n[q] * g.off[q];
+        }
+        for (int q = 0; q < 3 * d; ++q) {
+            const int v = p.sc.faces[3 * row.seq[q / 3] + q % 3];
+            if (!vertex_wanted(p, v)) continue;
+            bool seen = false;
+            for (int u = 0; u < q; ++u) seen = seen || p.sc.faces[3 * row.seq[u / 3] + u % 3] == v;
+            if (seen) continue;
+            V3<double> sum = fg[q / 3][q % 3];
+            for (int u = q + 1; u < 3 * d; ++u)
+                if (p.sc.faces[3 * row.seq[u / 3] + u % 3] == v) sum = sum + fg[u / 3][u % 3];
+            put3(gid_vertex(v, 0), sum);
+        }
+    }
+    if (p.want & kWantMaterials) {
+        for (int q = 0; q < d; ++q) {
+            const int m = p.sc.face_material[row.seq[q]];
+            bool seen = false;
+            for (int u = 0; u < q; ++u) seen = seen || p.sc.face_material[row.seq[u]] == m;
+            if (seen) continue;
+            double eps = g.eps[q], sig = g.sig[q];
+            for (int u = q + 1; u < d; ++u)
+                if (p.sc.face_material[row.seq[u]] == m) {
+                    eps += g.eps[u];
+                    sig += g.sig[u];
+                }
+            put(p.base_meps + m, eps);
+            put(p.base_msig + m, sig);
+        }
     }
 }
 
