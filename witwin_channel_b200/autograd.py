@@ -142,8 +142,12 @@ def _differentiable_inputs(scene, compiled, freqs_t: torch.Tensor, device) -> di
     """The scene values the solve is differentiated in: vertices (V,3), per
     frequency material and layer eps_r / sigma_e (NF,M) and (NF,L), the
     frequencies (NF,), Tx positions (T,3) and point-receiver positions (R,3)."""
-    verts = [st.vertices.reshape(-1, 3).to(device=device, dtype=torch.float64) for st in scene.structures]
-    V = torch.cat(verts) if verts else torch.zeros((0, 3), dtype=torch.float64, device=device)
+    verts = [st.vertices.reshape(-1, 3) for st in scene.structures]
+    if len({(v.device, v.dtype) for v in verts}) > 1:
+        verts = [v.to(device=device, dtype=torch.float64) for v in verts]
+    # joined where they live, then one copy (one per structure otherwise)
+    V = torch.cat(verts).to(device=device, dtype=torch.float64) if verts else \
+        torch.zeros((0, 3), dtype=torch.float64, device=device)
     eps, sig, leps, lsig = [], [], [], []
     layer_counts = []
     for f in range(freqs_t.shape[0]):
@@ -164,8 +168,8 @@ def _differentiable_inputs(scene, compiled, freqs_t: torch.Tensor, device) -> di
         rx = torch.stack([r.position.reshape(3).to(device=device, dtype=torch.float64) for r in rxs]) if rxs else \
             torch.zeros((0, 3), dtype=torch.float64, device=device)
     # differentiate only the vertices of structures whose vertex tensor takes gradients
-    mask = torch.cat([torch.full((st.vertices.reshape(-1, 3).shape[0],), int(bool(st.vertices.requires_grad)),
-                                 dtype=torch.uint8) for st in scene.structures]).to(device) if verts else None
+    mask = torch.tensor([int(bool(st.vertices.requires_grad)) for st in scene.structures], dtype=torch.uint8) \
+        .repeat_interleave(torch.tensor([v.shape[0] for v in verts])).to(device) if verts else None
     return {"vertices": V, "vertex_mask": mask, "eps_r": torch.stack(eps), "sigma_e": torch.stack(sig),
             "layer_eps_r": torch.stack(leps), "layer_sigma_e": torch.stack(lsig),
             "frequency": freqs_t.to(dtype=torch.float64), "tx": tx, "rx": rx, "layer_counts": layer_counts}

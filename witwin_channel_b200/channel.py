@@ -35,8 +35,7 @@ def cfr(paths, frequencies, *, num_tx: int, num_rx: int, normalize_delays: bool 
     if K < 1:
         raise ValueError("frequencies must not be empty")
     device = paths.tx_id.device
-    freqs = frequencies.to(device=device, dtype=torch.float64).contiguous()
-    f_host = freqs.cpu()
+    f_host = frequencies.detach().to(device="cpu", dtype=torch.float64).contiguous()
     df = 0.0
     if K > 1:
         steps = f_host[1:] - f_host[:-1]
@@ -44,11 +43,19 @@ def cfr(paths, frequencies, *, num_tx: int, num_rx: int, normalize_delays: bool 
             df = float(steps[0])
     elif K == 1:
         df = 1.0  # a single subcarrier: any step works
+    # only an uneven grid is read on the device (an upload from pageable memory
+    # waits for the work queued before it)
+    freqs = frequencies.to(device=device, dtype=torch.float64).contiguous() if df == 0.0 else None
     n = int(paths.tx_id.shape[0])
     if n > 1:
+        # checked on the device; read below, after the spectrum's launch, so the
+        # host does not wait with an idle device (an unordered table's spectrum
+        # stays within its buffers and is dropped)
         key = paths.rx_id.long() * max(int(num_tx), 1) + paths.tx_id.long()
-        if bool((key[1:] < key[:-1]).any()):
-            raise ValueError("paths must be in the canonical (rx, tx) order of an exported path table")
+        unordered = torch.empty((), dtype=torch.bool, pin_memory=True)
+        unordered.copy_((key[1:] < key[:-1]).any(), non_blocking=True)
+        checked = torch.cuda.Event()
+        checked.record()
     out = torch.empty((num_tx, num_rx, K), dtype=torch.complex64, device=device)
     a = _coefficients(paths).contiguous()
     lib = _native.load()
@@ -64,6 +71,10 @@ def cfr(paths, frequencies, *, num_tx: int, num_rx: int, normalize_delays: bool 
                     _native.ptr(ws), ws.numel(), _native.stream_handle(device)),
         "wcb_cfr",
     )
+    if n > 1:
+        checked.synchronize()
+        if bool(unordered):
+            raise ValueError("paths must be in the canonical (rx, tx) order of an exported path table")
     return out
 
 
