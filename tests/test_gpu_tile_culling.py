@@ -5,7 +5,7 @@ triangle across the whole shaft).  The same receivers in shuffled order fill
 their tiles with far-apart points, whose bounds span the scene and reject
 next to nothing, so both orders must give the same rows bit for bit.  The
 sizes take each number of warps per tile (8 below 1,024 tiles, 4 below 16,384,
-then 1, where eight tiles share a first diffraction test), with ragged edges."""
+then 1), with ragged edges."""
 
 from __future__ import annotations
 
@@ -40,7 +40,7 @@ def _rows(compiled, ep, mats, depth, rx_of):
     (1, 1, 12, 2, 2.0),        # one receiver
     (37, 29, 16, 3, 4.1),      # 8 warps per tile, ragged in both directions
     (189, 181, 40, 2, 1.9),    # 4 warps per tile
-    (733, 719, 9, 1, 0.21),    # 1 warp per tile, strips of eight tiles
+    (733, 719, 9, 1, 0.21),    # 1 warp per tile
 ])
 def test_grid_rows_equal_shuffled_points(rows, cols, boxes, depth, spacing):
     layout = city_layout(boxes, 11)

@@ -74,10 +74,10 @@ WCB_D V3<float> rx_point(const MainParams& p, int r) {
     return v3(p.rx_pos[3 * r], p.rx_pos[3 * r + 1], p.rx_pos[3 * r + 2]);
 }
 
-// number of 32-cell tiles per transmitter
+// number of tiles per transmitter
 WCB_HD long long tiles_per_tx(const MainParams& p) {
     if (p.rx_kind == 1) return (long long)((p.grid_rows + 7) / 8) * ((p.grid_cols + 3) / 4);
-    return (p.num_rx + 31) / 32;
+    return (p.num_rx + p.tile_cells - 1) / p.tile_cells;
 }
 
 // cell of (tile, lane); false for lanes past the grid edge
@@ -96,8 +96,8 @@ WCB_D bool tile_cell(const MainParams& p, long long tile_global, int lane, int* 
         *r = row * p.grid_cols + col;
         return true;
     }
-    const long long r64 = tile * 32 + lane;
-    if (r64 >= p.num_rx) return false;
+    const long long r64 = tile * p.tile_cells + lane;
+    if (lane >= p.tile_cells || r64 >= p.num_rx) return false;
     *r = int(r64);
     return true;
 }
@@ -878,13 +878,7 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
     const bool active = tile_cell(p, tile, lane, &t, &r);
     const long long per_tx = tiles_per_tx(p);
     const int tw = int(tile / per_tx);
-    // one tile per warp: the block's eight tiles (a strip of neighbours) share a
-    // first test when they have the same transmitter, so a shaft that one
-    // triangle blocks for the whole strip costs one traversal instead of eight
-    const long long first_tile = (long long)blockIdx.x * kSplitWarps;
-    const bool strip = tile_warps == 1 && first_tile / per_tx == (first_tile + kSplitWarps - 1) / per_tx &&
-                       first_tile + kSplitWarps <= per_tx * p.num_tx;
-    if (tw >= p.num_tx) return;  // whole groups; never in a strip
+    if (tw >= p.num_tx) return;  // whole groups
     t = tw;
     const SceneDev& sc = p.sc;
     int* err = p.status;
@@ -907,54 +901,19 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
         if (lane == 0) bounds = tb;
     }
     const int width = grp.warps * 32;
-    __shared__ int strip_edges[kSplitBlock], strip_n;
-    const int span = strip ? kSplitBlock : width;
-    int m = 0, i0 = 0;
-    for (int jb = j0; jb < jend || i0 < m;) {
-        if (strip && i0 >= m) {
-            // the strip's next 256 edges
-            __syncthreads();
-            if (threadIdx.x == 0) strip_n = 0;
-            __syncthreads();
-            const int js = jb + threadIdx.x;
-            if (js < jend) {
-                TileBounds sb = all_bounds[0];
-                for (int w = 1; w < kSplitWarps; ++w)
-                    for (int k = 0; k < 3; ++k) {
-                        sb.lo[k] = fminf(sb.lo[k], all_bounds[w].lo[k]);
-                        sb.hi[k] = fmaxf(sb.hi[k], all_bounds[w].hi[k]);
-                    }
-                ++rays;
-                if (edge_shaft_blocked(sc, list[js], S, sb, stack)) {
-                    for (int w = 0; w < kSplitWarps; ++w) vis_words[(first_tile + w) * chunk + (js - j0)] = 0u;
-                } else {
-                    strip_edges[atomicAdd(&strip_n, 1)] = js;
-                }
-            }
-            __syncthreads();
-            m = strip_n;
-            i0 = 0;
-            jb += span;
-            if (m == 0) continue;
-        } else if (!strip) {
-            m = min(span, jend - jb);
-            i0 = 0;
-        }
+    for (int jb = j0; jb < jend; jb += width) {
         if (grp.rank == 0 && lane == 0) num_open = 0;
         grp.sync();
         // one edge per thread: a pair whose Q -> tile shaft one triangle blocks
         // has no visible cell
-        const int per = (min(m - i0, width) + grp.warps - 1) / grp.warps;
-        const int at = i0 + grp.rank * per + lane;
-        if (lane < per && at < m) {
-            const int jt = strip ? strip_edges[at] : jb + at;
+        const int per = (min(jend - jb, width) + grp.warps - 1) / grp.warps;
+        const int jt = jb + grp.rank * per + lane;
+        if (lane < per && jt < jend) {
             ++rays;
             const bool closed = edge_shaft_blocked(sc, list[jt], S, bounds, stack);
             if (closed) vis_words[tile * chunk + (jt - j0)] = 0u;
             else open_edges[atomicAdd(&num_open, 1)] = jt;
         }
-        i0 += width;
-        if (!strip) jb += span;
         grp.sync();
         const int n = num_open;
         for (int i = grp.rank; i < n; i += grp.warps) {

@@ -27,6 +27,7 @@ struct MainParams {
     SceneDev sc;
     int num_tx, num_rx;
     int rx_kind;
+    int tile_cells;  // point receivers per tile: 32, or 1 when they are few
     const float* rx_pos;
     float grid_origin[3], grid_x[3], grid_y[3];
     int grid_rows, grid_cols;
