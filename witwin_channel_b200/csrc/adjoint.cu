@@ -361,7 +361,7 @@ int wcb_rows_vjp(const wcb_scene* scene, const wcb_solve_desc* desc, const wcb_m
             switch (cids[r]) {
                 case 0: wcb::adj::k_vjp_rows<wcb::adj::kLanes, 0><<<g, wcb::adj::kBlock, 0, s>>>(p); break;
                 case 1: wcb::adj::k_vjp_reflection<<<g, wcb::adj::kBlock, 0, s>>>(p); break;
-                case 5: wcb::adj::k_vjp_rows<wcb::adj::kLanes, 5><<<g, wcb::adj::kBlock, 0, s>>>(p); break;
+                case 5: wcb::adj::launch_vjp_transmission(p, s); break;
                 default: {
                     wcb::ProfileState& prof = wcb::profile_state();
                     cudaEvent_t e0 = nullptr, e1 = nullptr;

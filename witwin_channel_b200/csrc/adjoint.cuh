@@ -676,6 +676,7 @@ static __global__ void __launch_bounds__(kBlock) k_vjp_reflection(AdjParams p) {
 }
 
 void launch_vjp_diffraction(const AdjParams& p, cudaStream_t s);
+void launch_vjp_transmission(const AdjParams& p, cudaStream_t s);
 void fill_params(AdjParams& p, const SceneHandle* h, const wcb_solve_desc* desc, const wcb_materials* materials,
                  int freq_index, const void* rows, const int64_t* selected, long long K, const int64_t* layout);
 
