@@ -355,19 +355,20 @@ WCB_D bool project_bounds(float nx, float ny, float nz, float off, float ix, flo
 // back bounce by bounce, each cut to its group's box.
 WCB_D bool tile_may_reflect(const MainParams& p, const TileBounds& b, long long base, int c, int d) {
     float lo[3] = {b.lo[0], b.lo[1], b.lo[2]}, hi[3] = {b.hi[0], b.hi[1], b.hi[2]};
-    const float4 pl = __ldg(p.chain_pre + (base + c) * 2);
-    const float4 im = __ldg(p.chain_pre + (base + c) * 2 + 1);
-    if (!project_bounds(pl.x, pl.y, pl.z, pl.w, im.x, im.y, im.z, p.sc.group_box + 6 * __float_as_int(im.w), lo, hi))
-        return false;
+    float4 pl = __ldg(p.chain_pre + (base + c) * 2);
+    float4 im = __ldg(p.chain_pre + (base + c) * 2 + 1);
+    int group = __float_as_int(im.w);
     const long long row = base + (long long)c * d;
-    for (int k = d - 2; k >= 0; --k) {
+#pragma unroll 1
+    for (int k = d - 1;;) {
+        if (!project_bounds(pl.x, pl.y, pl.z, pl.w, im.x, im.y, im.z, p.sc.group_box + 6 * group, lo, hi)) return false;
+        if (--k < 0) return true;
         const double* q = p.chain_planes + (row + k) * 4;
         const double* i = p.chain_images + (row + k) * 3;
-        if (!project_bounds(float(q[0]), float(q[1]), float(q[2]), float(q[3]), float(i[0]), float(i[1]), float(i[2]),
-                            p.sc.group_box + 6 * p.chain_groups[row + k], lo, hi))
-            return false;
+        pl = make_float4(float(q[0]), float(q[1]), float(q[2]), float(q[3]));
+        im = make_float4(float(i[0]), float(i[1]), float(i[2]), 0.f);
+        group = p.chain_groups[row + k];
     }
-    return true;
 }
 
 // Does one triangle block the last leg (hit on the last plane -> receiver) of
@@ -474,7 +475,10 @@ WCB_D int queue_pop_faces(int* q, int* qfaces, int size, int n, int lane) {
 // what is left from 1.8 to 1.3 per candidate.  Before and after, on one B200:
 // canyon 1.25 -> 0.80 ms, four-transmitter batch 15.4 -> 8.0 ms, 2048-box city
 // (1024^2 cells, depth 5) 167 -> 25-30 ms, a 90 x 70 town with 25,760
-// exhaustive chains 4.0 -> 0.6 ms.
+// exhaustive chains 4.0 -> 0.6 ms.  What is left is the visibility traversal
+// (0.4 ms of the canyon) and fetch: rolled loops and one copy of each helper
+// took 0.83 -> 0.72 ms, dealing the last visible paths of a group out again in
+// full batches 0.72 -> 0.66-0.70 ms (no-instruction stalls 5.6 -> 2.0 per issue).
 template <typename T, int NF>
 __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect(MainParams p, int stack_depth,
                                                                                            int tile_warps) {
@@ -550,6 +554,7 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
                 V3<T> incident = safe_normalize(cast3<T>(hits[0]) - prev, v3<T>(T(0), T(0), T(1)));
                 C3<T> value = c3_from_real(transverse(incident, tx_pol));
                 V3<T> outgoing = incident;
+#pragma unroll 1
                 for (int k = 0; k < d; ++k) {
                     const V3<T> hit = cast3<T>(hits[k]);
                     incident = safe_normalize(hit - prev, outgoing);
@@ -642,6 +647,7 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
             const double* images = p.chain_images + (base + (long long)c * d) * 3;
             // hit k and its face, from the last bounce back (no hit array)
             V3<double> x = v3<double>(rx, ry, rz);
+#pragma unroll 1
             for (int k = d - 1; k >= 0 && ok; --k) {
                 ok = back_project_step(x, planes, images, k);
                 const int f = ok ? resolve_in_group(sc, groups[k], x) : -1;
@@ -701,7 +707,8 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
             }
         };
         enter_depth();
-        bool last;
+        // FP64 keeps each warp's paths (the grouping below)
+        bool last, merged = grp.warps == 1 || sizeof(T) == 8;
         do {
             // the next candidates that the tile may see, one test per thread
             listed = 0;
@@ -750,6 +757,7 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
                 else if (!last) break;
                 else if (qa > 0) step = 1;
                 else if (qb > 0) step = 2;
+                else if (!merged) step = 4;
                 else if (qf > 0) step = 3;
                 else break;
                 if (step == 0) {
@@ -763,8 +771,34 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
                     process_a(qa < 32 ? qa : 32);
                 } else if (step == 2) {
                     process_b(qb < 32 ? qb : 32);
-                } else {
+                } else if (step == 3) {
                     process_f(qf < 32 ? qf : 32);
+                } else {
+                    // the group's last visible paths (fewer than 32 a warp) dealt
+                    // out again in full batches: the field stage is long straight
+                    // code, and every extra pass through it flushes the others'
+                    // instructions
+                    merged = true;
+                    int item[3], faces[kMaxDepth];
+                    for (int k = 0; k < 3; ++k) item[k] = lane < qf ? sh->qf[3 * lane + k] : 0;
+#pragma unroll
+                    for (int k = 0; k < kMaxDepth; ++k) faces[k] = lane < qf ? sh->qff[kMaxDepth * lane + k] : 0;
+                    if (lane == 0) warp_n[grp.rank] = qf;
+                    grp.sync();
+                    int at = lane, total = 0;
+                    for (int w = 0; w < grp.warps; ++w) {
+                        if (w < grp.rank) at += warp_n[w];
+                        total += warp_n[w];
+                    }
+                    if (lane < qf) {
+                        ReflShared<NF>* to = sh - grp.rank + (at >> 5);
+                        const int slot = at & 31;
+                        for (int k = 0; k < 3; ++k) to->qf[3 * slot + k] = item[k];
+#pragma unroll
+                        for (int k = 0; k < kMaxDepth; ++k) to->qff[kMaxDepth * slot + k] = faces[k];
+                    }
+                    grp.sync();
+                    qf = min(max(total - 32 * grp.rank, 0), 32);
                 }
             }
             grp.sync();

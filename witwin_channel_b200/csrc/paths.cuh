@@ -41,6 +41,7 @@ WCB_D int resolve_in_group(const SceneDev& sc, int g, V3<double> p) {
     const float* bx = sc.group_box + 6 * g;
     if (p.x < bx[0] || p.y < bx[1] || p.z < bx[2] || p.x > bx[3] || p.y > bx[4] || p.z > bx[5]) return -1;
     const int beg = sc.group_member_off[g], end = sc.group_member_off[g + 1];
+#pragma unroll 1
     for (int i = beg; i < end; ++i) {
         const int f = sc.group_members[i];
         if (point_in_face(sc, f, p)) return f;
@@ -68,6 +69,7 @@ WCB_D bool back_project_step(V3<double>& x, const double* planes, const double* 
 
 WCB_D bool back_project(V3<double> R, const double* planes, const double* images, int depth, V3<double>* hits) {
     V3<double> x = R;
+#pragma unroll 1
     for (int k = depth - 1; k >= 0; --k) {
         if (!back_project_step(x, planes, images, k)) return false;
         hits[k] = x;
@@ -83,6 +85,7 @@ WCB_D bool back_project_segment(V3<double> S, V3<double> R, const double* planes
     V3<double> x = R;
     *a = S;
     *b = R;
+#pragma unroll 1
     for (int k = depth - 1; k >= 0 && k >= s - 1; --k) {
         if (!back_project_step(x, planes, images, k)) return false;
         if (k == s) *b = x;

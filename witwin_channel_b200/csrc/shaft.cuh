@@ -116,8 +116,9 @@ WCB_D bool shaft_blocked(const SceneDev& sc, V3<float> p0, V3<float> p1, const I
                 have_next = true;
             }
         }
+#pragma unroll 1
         for (int k = 0; k < leaves; ++k) {
-            const int slot = ~leaf[k];
+            const int slot = ~(k == 0 ? leaf[0] : leaf[1]);
             const float4 a = __ldg(sc.tri + 3 * slot + 0);
             const float4 b = __ldg(sc.tri + 3 * slot + 1);
             const float4 c = __ldg(sc.tri + 3 * slot + 2);

@@ -97,6 +97,11 @@ WCB_D bool box_hit(const Ray<G>& r, G lx, G ly, G lz, G hx, G hy, G hz, G tmax, 
 WCB_D float edge_fn(float a, float b, float c, float d) { return __fsub_rn(__fmul_rn(a, b), __fmul_rn(c, d)); }
 WCB_D double edge_fn(double a, double b, double c, double d) { return __dsub_rn(__dmul_rn(a, b), __dmul_rn(c, d)); }
 
+// The same in FP64, for edge functions that are zero in FP32 (rare: out of line).
+__device__ __noinline__ inline double edge_fn64(float a, float b, float c, float d) {
+    return edge_fn(double(a), double(b), double(c), double(d));
+}
+
 // Watertight ray/triangle test.  Returns t (ray parameter) or +inf.
 template <typename G>
 WCB_D G tri_hit(const Ray<G>& r, float4 a4, float4 b4, float4 c4) {
@@ -118,9 +123,9 @@ WCB_D G tri_hit(const Ray<G>& r, float4 a4, float4 b4, float4 c4) {
     G V = edge_fn(Ax, Cy, Ay, Cx_);
     G W = edge_fn(Bx, Ay, By, Ax);
     if (sizeof(G) == 4 && (U == G(0) || V == G(0) || W == G(0))) {
-        U = G(edge_fn(double(Cx_), double(By), double(Cy), double(Bx)));
-        V = G(edge_fn(double(Ax), double(Cy), double(Ay), double(Cx_)));
-        W = G(edge_fn(double(Bx), double(Ay), double(By), double(Ax)));
+        U = G(edge_fn64(float(Cx_), float(By), float(Cy), float(Bx)));
+        V = G(edge_fn64(float(Ax), float(Cy), float(Ay), float(Cx_)));
+        W = G(edge_fn64(float(Bx), float(Ay), float(By), float(Ax)));
     }
     const G inf = sizeof(G) == 4 ? G(__int_as_float(0x7f800000)) : G(__longlong_as_double(0x7ff0000000000000LL));
     if ((U < G(0) || V < G(0) || W < G(0)) && (U > G(0) || V > G(0) || W > G(0))) return inf;
@@ -187,13 +192,20 @@ WCB_D bool traverse(const SceneDev& sc, Ray<G> r, const Ignore& ig, int* stack, 
         bool h1 = box_hit(r, G(b.z), G(b.w), G(c.x), G(c.y), G(c.z), G(c.w), tmax, &n1);
         int next = -1;
         bool have_next = false;
-        if (h0 && d.x < 0) {
-            if (leaf(d.x)) return true;
-            h0 = false;
+        // leaves among the children, in order, through one inlined copy of the
+        // triangle test (the kernels that traverse are bound by instruction fetch)
+        int first = h0 && d.x < 0 ? d.x : 0, second = h1 && d.y < 0 ? d.y : 0;
+        h0 = h0 && d.x >= 0;
+        h1 = h1 && d.y >= 0;
+        if (first == 0) {
+            first = second;
+            second = 0;
         }
-        if (h1 && d.y < 0) {
-            if (leaf(d.y)) return true;
-            h1 = false;
+#pragma unroll 1
+        while (first != 0) {
+            if (leaf(first)) return true;
+            first = second;
+            second = 0;
         }
         if (h0 && h1) {
             const bool first0 = n0 <= n1;
