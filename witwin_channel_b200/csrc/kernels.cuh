@@ -707,8 +707,7 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
             }
         };
         enter_depth();
-        // FP64 keeps each warp's paths (the grouping below)
-        bool last, merged = grp.warps == 1 || sizeof(T) == 8;
+        bool last, merged = false;
         do {
             // the next candidates that the tile may see, one test per thread
             listed = 0;
@@ -774,11 +773,14 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
                 } else if (step == 3) {
                     process_f(qf < 32 ? qf : 32);
                 } else {
-                    // the group's last visible paths (fewer than 32 a warp) dealt
-                    // out again in full batches: the field stage is long straight
-                    // code, and every extra pass through it flushes the others'
-                    // instructions
+                    // the block's warps enter the field stage together: it is long
+                    // straight code, fetched once for all of them.  The group's
+                    // last visible paths (fewer than 32 a warp) are dealt out again
+                    // in full batches; FP64 keeps each warp's paths (the grouping
+                    // above).
                     merged = true;
+                    __syncthreads();
+                    if (grp.warps == 1 || sizeof(T) == 8) continue;
                     int item[3], faces[kMaxDepth];
                     for (int k = 0; k < 3; ++k) item[k] = lane < qf ? sh->qf[3 * lane + k] : 0;
 #pragma unroll
@@ -1134,10 +1136,20 @@ __global__ void __launch_bounds__(kSplitBlock, 2) k_diffract_utd(MainParams p, i
         jj += first;
         seen += before;
     }
-    // one loop walks the words and drives the queue so the UTD stage is
-    // inlined once
-    while (true) {
-        if (jj < nw && seen < hi) {
+    // The block's warps take their batches in step: the UTD stage is long
+    // straight code, and warps that drift apart in it flush each other's
+    // instructions (no-instruction stalls 3.8 -> 0.5 per issue; one B200, before
+    // and after: canyon 0.36 -> 0.32 ms, FP64 canyon 0.24 -> 0.16, four
+    // transmitters and frequencies 7.4 -> 5.7).  Groups without a tile have left
+    // the block, which the barrier allows.
+    __shared__ int all_batches;
+    if (threadIdx.x == 0) all_batches = 0;
+    __syncthreads();
+    if (lane == 0) atomicMax(&all_batches, (hi - lo + 31) / 32);
+    __syncthreads();
+    const int batches = all_batches;
+    for (int batch = 0; batch < batches; ++batch) {
+        while (qv < 32 && jj < nw && seen < hi) {
             const unsigned word = words[jj];
             const int idx = seen + __popc(word & lanemask_lt());
             const bool mine = ((word >> lane) & 1u) && idx >= lo && idx < hi;
@@ -1145,13 +1157,12 @@ __global__ void __launch_bounds__(kSplitBlock, 2) k_diffract_utd(MainParams p, i
             seen += __popc(word);
             ++jj;
         }
-        const bool drained = !(jj < nw && seen < hi);
-        if (qv >= 32 || (drained && qv > 0)) {
+        __syncthreads();
+        if (qv > 0) {
             const int n = qv < 32 ? qv : 32;
             process_v(n);
             qv = queue_pop(sh->qv, qv, n, lane);
         }
-        if (drained && qv == 0) break;
     }
     // fixed-order reduction of the warps' partial sums, one write per cell
     for (int f = 0; f < NF; ++f) {
