@@ -24,6 +24,9 @@ constexpr int kCompBlock = kWarpsPerBlock * 32;
 constexpr int kSplitWarps = 8;                 // reflection/diffraction: one tile per block,
 constexpr int kSplitBlock = kSplitWarps * 32;  // its candidates interleaved over 8 warps
 constexpr int kQueueCap = 64;
+constexpr int kEdgeSpan = 128;   // diffraction edges per warp between two lists of open pairs
+constexpr int kEdgeRefill = 8;   // idle lanes that take new edges
+constexpr int kEdgeDescend = 8;  // descending lanes below which the waiting lanes' leaves are tested
 constexpr int kCandCap = 64;  // reflection candidates listed per round and warp
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -845,12 +848,13 @@ struct DiffShared {
 // runs at twice the occupancy of the field kernel and neither competes with
 // the other for instruction cache.
 
-// Does one triangle block every Q -> Rx segment between the edge and a tile?
+// The shaft of every Q -> Rx segment between the edge and a tile, with its
+// centre line's near end (the far end is the middle of the bounds).
 // The clamped stationary point moves along the edge with the receiver:
 // t* = ts + (tr - ts) rs / (rs + rr) is monotone in the receiver's edge
 // coordinate tr and, with the sign of tr - ts, in its edge distance rr, so its
 // range over the tile's bounds is spanned by the ends of their ranges.
-WCB_D bool edge_shaft_blocked(const SceneDev& sc, int edge, V3<double> S, const TileBounds& b, int* stack) {
+WCB_D V3<float> edge_shaft(const SceneDev& sc, int edge, V3<double> S, const TileBounds& b, Shaft& s, Ignore& ig) {
     const EdgeDev& ed = sc.edges[edge];
     const V3<float> c = v3(float(ed.pos[0]), float(ed.pos[1]), float(ed.pos[2]));
     const V3<float> e = v3(float(ed.dir[0]), float(ed.dir[1]), float(ed.dir[2]));
@@ -874,7 +878,6 @@ WCB_D bool edge_shaft_blocked(const SceneDev& sc, int edge, V3<double> S, const 
     const float q_lo = fminf(fmaxf(t_lo, -hl), hl), q_hi = fminf(fmaxf(t_hi, -hl), hl);
     const V3<float> bias = v3(float(ed.bisector[0]), float(ed.bisector[1]), float(ed.bisector[2])) *
                            float(kDiffractionRayBias);
-    Shaft s;
     s.a[0] = c + e * q_lo + bias;
     s.a[1] = c + e * q_hi + bias;
     s.na = q_hi > q_lo ? 2 : 1;
@@ -884,10 +887,10 @@ WCB_D bool edge_shaft_blocked(const SceneDev& sc, int edge, V3<double> S, const 
     }
     s.size = size;
     s.side = 0.f;
-    Ignore ig = ignore_none();
+    ig = ignore_none();
     ig.f0 = ed.face0;
     ig.f1 = ed.face1;
-    return shaft_blocked(sc, (s.a[0] + s.a[1]) * 0.5f, mid, ig, s, stack);
+    return (s.a[0] + s.a[1]) * 0.5f;
 }
 
 // Visibility words of edges [j0, j0 + chunk) of each tile's transmitter: bit
@@ -895,13 +898,16 @@ WCB_D bool edge_shaft_blocked(const SceneDev& sc, int edge, V3<double> S, const 
 // for that lane's cell, Q the clamped stationary point on the edge moved by
 // kDiffractionRayBias along its exterior bisector.
 //
-// Issue bound (68-74 %).  One thread first tries to close a whole (tile, edge)
+// Issue bound (68-78 %).  One thread first tries to close a whole (tile, edge)
 // pair with one triangle (shaft.cuh), so a warp settles 32 pairs with one
 // divergent traversal where it took 32 coherent ones; only open pairs are
 // traced per cell, the receiver's leg first (49 % of the canyon's are clear,
 // against 88 % of the transmitter's).  It closes 77 % of the canyon's pairs and
 // 98.5 % of the 2048-box city's.  Before and after, on one B200: canyon 0.44 ->
-// 0.30-0.34 ms, four-transmitter batch 5.35 -> 3.1 ms, city 245 -> 60 ms.
+// 0.30-0.36 ms, four-transmitter batch 5.35 -> 3.2 ms, city 245 -> 57 ms.  Most of
+// that is the city's 57 M shaft searches: run as plain per-lane loops their
+// triangle tests were taken by 6 lanes of 32 (64 ms); descending together and
+// testing together with idle lanes refilled takes 57 (thresholds 4 to 16: 57 to 65).
 template <typename T>
 __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, int tile_warps, int j0, int chunk,
                                                                  unsigned* vis_words) {
@@ -928,27 +934,58 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
     const V3<double> R = cast3<double>(Rf);
     unsigned long long rays = 0;
     __shared__ TileBounds all_bounds[kSplitWarps];
-    __shared__ int all_open[kSplitBlock], all_n[kSplitWarps];
+    __shared__ int all_open[kSplitWarps * kEdgeSpan], all_n[kSplitWarps];
     TileBounds& bounds = all_bounds[grp.index];
-    int* open_edges = all_open + grp.index * grp.warps * 32;
+    int* open_edges = all_open + grp.index * grp.warps * kEdgeSpan;
     int& num_open = all_n[grp.index];
     if (grp.rank == 0) {
         const TileBounds tb = tile_bounds(Rf, active);
         if (lane == 0) bounds = tb;
     }
-    const int width = grp.warps * 32;
+    const int width = grp.warps * kEdgeSpan;
     for (int jb = j0; jb < jend; jb += width) {
         if (grp.rank == 0 && lane == 0) num_open = 0;
         grp.sync();
-        // one edge per thread: a pair whose Q -> tile shaft one triangle blocks
-        // has no visible cell
+        // One edge per lane: a pair whose Q -> tile shaft one triangle blocks has
+        // no visible cell.  The searches differ in length, so a lane that is done
+        // takes the warp's next edge once enough lanes are idle.
         const int per = (min(jend - jb, width) + grp.warps - 1) / grp.warps;
-        const int jt = jb + grp.rank * per + lane;
-        if (lane < per && jt < jend) {
-            ++rays;
-            const bool closed = edge_shaft_blocked(sc, list[jt], S, bounds, stack);
-            if (closed) vis_words[tile * chunk + (jt - j0)] = 0u;
-            else open_edges[atomicAdd(&num_open, 1)] = jt;
+        int next = jb + grp.rank * per;
+        const int end = min(next + per, jend);
+        ShaftSearch q;
+        Shaft sh;
+        Ignore ig = ignore_none();
+        int jt = -1;
+        while (true) {
+            const unsigned idle = __ballot_sync(kFull, jt < 0);
+            if (next < end && __popc(idle) >= kEdgeRefill) {
+                const int mine = next + __popc(idle & lanemask_lt());
+                if (jt < 0 && mine < end) {
+                    jt = mine;
+                    const V3<float> near_end = edge_shaft(sc, list[jt], S, bounds, sh, ig);
+                    q.start(sc, near_end, v3(0.5f * (bounds.lo[0] + bounds.hi[0]), 0.5f * (bounds.lo[1] + bounds.hi[1]),
+                                             0.5f * (bounds.lo[2] + bounds.hi[2])));
+                    ++rays;
+                }
+                next += __popc(idle);
+            } else if (idle == kFull) {
+                break;
+            }
+            // descend until most lanes stand at a leaf, then test together
+#pragma unroll 1
+            for (int it = 0; it < 16; ++it) {
+                const bool go = jt >= 0 && q.leaf0 == 0 && q.next != ShaftSearch::kNone;
+                if (__popc(__ballot_sync(kFull, go)) < kEdgeDescend) break;
+                if (go) q.node(sc, stack);
+            }
+            if (jt >= 0) {
+                bool closed = false;
+                if (q.leaf0 != 0) closed = q.test(sc, ig, sh);
+                else if (q.next != ShaftSearch::kNone) q.node(sc, stack);
+                if (closed) vis_words[tile * chunk + (jt - j0)] = 0u;
+                else if (q.done()) open_edges[atomicAdd(&num_open, 1)] = jt;
+                if (closed || q.done()) jt = -1;
+            }
         }
         grp.sync();
         const int n = num_open;

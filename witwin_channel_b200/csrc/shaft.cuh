@@ -84,53 +84,72 @@ WCB_D bool triangle_cuts_shaft(const Shaft& s, V3<float> v0, V3<float> v1, V3<fl
     return true;
 }
 
-// Any triangle outside `ig` on the segment p0 -> p1 (the shaft's centre line)
-// that cuts the whole shaft.
+// Search of the shaft's centre line for a triangle outside `ig` that cuts the
+// whole shaft, in resumable pieces: node() descends to the next leaves, test()
+// tries one leaf.  A warp that settles many shafts runs the two apart, so the
+// long triangle test is taken by many lanes at once, and a lane that is done
+// takes its next shaft.
+struct ShaftSearch {
+    V3<float> o, inv;
+    int next, sp;      // next node or (single-triangle scene) leaf; kNone when nothing is left
+    int leaf0, leaf1;  // leaves to try (0: none)
+    static constexpr int kNone = 0x7fffffff;
+
+    WCB_D void start(const SceneDev& sc, V3<float> p0, V3<float> p1) {
+        const Ray<float> r = make_ray<float>(p0, p1 - p0, 1e-6f, 1.f - 1e-6f);
+        o = r.o;
+        inv = r.inv;
+        sp = 0;
+        leaf1 = 0;
+        leaf0 = sc.root < 0 ? sc.root : 0;
+        next = sc.root < 0 ? kNone : sc.root;
+    }
+    WCB_D bool done() const { return leaf0 == 0 && next == kNone; }
+
+    WCB_D void node(const SceneDev& sc, int* stack) {
+        Ray<float> r;
+        r.o = o;
+        r.inv = inv;
+        r.tmin = 1e-6f;
+        const int stride = blockDim.x, lane = threadIdx.x;
+        float4 a, b, c;
+        int4 d;
+        load_node(sc.nodes, next, a, b, c, d);
+        float n0, n1;
+        const bool h0 = box_hit(r, a.x, a.y, a.z, a.w, b.x, b.y, 1.f - 1e-6f, &n0);
+        const bool h1 = box_hit(r, b.z, b.w, c.x, c.y, c.z, c.w, 1.f - 1e-6f, &n1);
+        const int l0 = h0 && d.x < 0 ? d.x : 0, l1 = h1 && d.y < 0 ? d.y : 0;
+        leaf0 = l0 ? l0 : l1;
+        leaf1 = l0 ? l1 : 0;
+        const bool in0 = h0 && d.x >= 0, in1 = h1 && d.y >= 0;
+        // a full stack drops the far child: it can only leave the shaft unsettled
+        if (in0 && in1 && sp < sc.stack_entries) stack[sp++ * stride + lane] = d.y;
+        if (in0 || in1) next = in0 ? d.x : d.y;
+        else next = sp > 0 ? stack[--sp * stride + lane] : kNone;
+    }
+
+    // Does the next leaf's triangle cut the shaft?
+    WCB_D bool test(const SceneDev& sc, const Ignore& ig, const Shaft& s) {
+        const int slot = ~leaf0;
+        leaf0 = leaf1;
+        leaf1 = 0;
+        const float4 a = __ldg(sc.tri + 3 * slot + 0);
+        const float4 b = __ldg(sc.tri + 3 * slot + 1);
+        const float4 c = __ldg(sc.tri + 3 * slot + 2);
+        return !ignored(ig, __float_as_int(a.w), __float_as_int(b.w)) &&
+               triangle_cuts_shaft(s, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z));
+    }
+};
+
 WCB_D bool shaft_blocked(const SceneDev& sc, V3<float> p0, V3<float> p1, const Ignore& ig, const Shaft& s, int* stack) {
     if (sc.num_faces == 0) return false;
-    const Ray<float> r = make_ray<float>(p0, p1 - p0, 1e-6f, 1.f - 1e-6f);
-    const int stride = blockDim.x, lane = threadIdx.x;
-    int sp = 0, node = sc.root;
-    while (true) {
-        int leaf[2], leaves = 0, next = 0;
-        bool have_next = false;
-        if (node < 0) {  // single-triangle scene
-            leaf[leaves++] = node;
-        } else {
-            float4 a, b, c;
-            int4 d;
-            load_node(sc.nodes, node, a, b, c, d);
-            float n0, n1;
-            const bool h0 = box_hit(r, a.x, a.y, a.z, a.w, b.x, b.y, r.tmax, &n0);
-            const bool h1 = box_hit(r, b.z, b.w, c.x, c.y, c.z, c.w, r.tmax, &n1);
-            if (h0 && d.x < 0) leaf[leaves++] = d.x;
-            if (h1 && d.y < 0) leaf[leaves++] = d.y;
-            const bool in0 = h0 && d.x >= 0, in1 = h1 && d.y >= 0;
-            if (in0 && in1) {
-                // a full stack drops the far child: it can only leave the shaft unsettled
-                if (sp < sc.stack_entries) stack[sp++ * stride + lane] = d.y;
-                next = d.x;
-                have_next = true;
-            } else if (in0 || in1) {
-                next = in0 ? d.x : d.y;
-                have_next = true;
-            }
-        }
-#pragma unroll 1
-        for (int k = 0; k < leaves; ++k) {
-            const int slot = ~(k == 0 ? leaf[0] : leaf[1]);
-            const float4 a = __ldg(sc.tri + 3 * slot + 0);
-            const float4 b = __ldg(sc.tri + 3 * slot + 1);
-            const float4 c = __ldg(sc.tri + 3 * slot + 2);
-            if (ignored(ig, __float_as_int(a.w), __float_as_int(b.w))) continue;
-            if (triangle_cuts_shaft(s, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z))) return true;
-        }
-        if (!have_next) {
-            if (sp == 0) return false;
-            next = stack[--sp * stride + lane];
-        }
-        node = next;
+    ShaftSearch q;
+    q.start(sc, p0, p1);
+    while (!q.done()) {
+        while (q.leaf0 == 0 && q.next != ShaftSearch::kNone) q.node(sc, stack);
+        if (q.leaf0 != 0 && q.test(sc, ig, s)) return true;
     }
+    return false;
 }
 
 }  // namespace wcb
