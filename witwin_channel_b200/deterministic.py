@@ -203,6 +203,12 @@ def _layout(values: torch.Tensor, rx: dict) -> torch.Tensor:
     return values.contiguous()
 
 
+def _layout_slots(values: torch.Tensor, rx: dict) -> torch.Tensor:
+    """:func:`_layout` of every slot of ``values`` (slots, T, R)."""
+    flat = _layout(values.reshape(values.shape[0] * values.shape[1], values.shape[2]), rx)
+    return flat.reshape(values.shape[0], values.shape[1], *flat.shape[1:])
+
+
 def _metadata(config: Config, counts: dict, path_count: int, launches: int, extra: dict) -> dict:
     components = {c: ("enabled" if c in config.components else "not_requested") for c in sorted(VALID_COMPONENTS)}
     if "transmission" in config.components:
@@ -303,9 +309,10 @@ def solve(scene: Any, config: Config, *, reference_frequency_hz, precision: str 
     field = cells.field[0]
     extra_components = tuple(n for n in _OPTIONAL_COMPONENTS if n in config.components)
     names = _BASE_COMPONENTS + extra_components
-    comp_power = {n: _layout(cells.comp_power[_SLOTS[n], 0], rx) for n in names}
-    comp_fields = {n: (_layout(cells.comp_field[_SLOTS[n], 0], rx) if config.return_field
-                       else torch.empty((0,), dtype=torch.complex64, device=device)) for n in names}
+    # the named slots are the first ones: laid out in one launch each for powers and fields
+    comp_power = dict(zip(names, _layout_slots(cells.comp_power[:len(names), 0], rx).unbind(0)))
+    comp_fields = dict(zip(names, _layout_slots(cells.comp_field[:len(names), 0], rx).unbind(0))) \
+        if config.return_field else {n: torch.empty((0,), dtype=torch.complex64, device=device) for n in names}
     exact = None
     if "diffraction" in config.components and rx["kind"] == "grid" and len(scene.receivers) == 1:
         exact = _layout(cells.diff_vec_power[0], rx)

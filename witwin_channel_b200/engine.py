@@ -82,7 +82,10 @@ def make_desc(ep: Endpoints, frequencies: list[float], components: int, max_dept
 
 def check_device_status(status: torch.Tensor) -> None:
     """Raise if a solve's device status word has a failure bit set (reads it: a sync)."""
-    st = int(status.item())
+    _raise_status(int(status.item()))
+
+
+def _raise_status(st: int) -> None:
     if st != 0:
         raise RuntimeError(f"native solve reported device status bits {st:#x} (bit 0: traversal stack overflow)")
 
@@ -154,9 +157,10 @@ def run_solve(compiled: CompiledScene, ep: Endpoints, mats: MaterialTables, freq
     _native.check(lib.wcb_solve_workspace_size(compiled.native.handle, ctypes.byref(desc), ctypes.byref(nbytes)),
                   "wcb_solve_workspace_size")
     ws = (workspace or _WORKSPACE).get(nbytes.value, device)
-    status = torch.zeros(1, dtype=torch.int32, device=device)
-    row_count = torch.zeros(1, dtype=torch.int64, device=device)
-    trans_overflow = torch.zeros(1, dtype=torch.int64, device=device)
+    counters = torch.zeros(3, dtype=torch.int64, device=device)  # one fill for the three words the solve reports
+    status = counters[0:1].view(torch.int32)[:1]
+    row_count = counters[1:2]
+    trans_overflow = counters[2:3]
     # row capacity: the caller's, else the last count seen on this scene (with
     # headroom), else 8 records per cell; a short buffer makes the solve run again
     hint = compiled.row_count_hint
@@ -183,11 +187,17 @@ def run_solve(compiled: CompiledScene, ep: Endpoints, mats: MaterialTables, freq
             continue
         _native.check(rc, "wcb_solve")
         break
-    if check_status:
+    n = 0
+    if want_rows:
+        # status and row count in one read
+        words = counters.tolist()
+        if check_status:
+            _raise_status(words[0])
+        n = int(words[1])
+    elif check_status:
         check_device_status(status)
     result = {"desc": desc, "keep": keep, "status": status, "workspace": ws, "transmission_overflow": trans_overflow}
     if want_rows:
-        n = int(row_count.item())
         result["rows"] = rows[:n]
         compiled.row_count_hint = max(n, compiled.row_count_hint)
     return result
