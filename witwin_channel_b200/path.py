@@ -27,6 +27,7 @@ from __future__ import annotations
 import ctypes
 import enum
 import math
+from collections import Counter
 from dataclasses import dataclass, replace
 from typing import Any
 
@@ -790,13 +791,14 @@ def _endpoint_factor(endpoints: list, directions: torch.Tensor, *, frequency_hz:
     (``directions[i]`` for ``endpoints[i]``): (endpoint, *batch, A).  Endpoints
     of one pattern kind are evaluated in one batch (a call per endpoint took 25
     launches each: 950 of the 1,263 launches of a 37-receiver solve); a custom
-    pattern's callable sees one endpoint's directions at a time, as do arrays
-    that live on different devices."""
+    pattern's callable sees one endpoint's directions at a time, and an object
+    that stands for many endpoints (a grid's points) keeps a batch of its own."""
 
+    uses = Counter(id(endpoint) for endpoint in endpoints)
     groups: dict[Any, list[int]] = {}
     for index, endpoint in enumerate(endpoints):
-        key = id(endpoint) if endpoint.pattern.kind == "custom" else (endpoint.pattern.kind,
-                                                                      endpoint.element_positions.device)
+        own = endpoint.pattern.kind == "custom" or uses[id(endpoint)] > 1
+        key = id(endpoint) if own else (endpoint.pattern.kind, endpoint.element_positions.device)
         groups.setdefault(key, []).append(index)
 
     def weights(members: list, sub: torch.Tensor) -> torch.Tensor:
