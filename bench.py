@@ -11,7 +11,8 @@ scene's concrete eps_r and sigma_e and every transmitter position.  Data are
 synthetic (seeded); no dataset is read.
 
 * ``value``: rays per second (segment visibility/penetration queries plus the
-  discovery bounces of every solve in the step) over the whole job, the L2
+  discovery bounces of every solve in the step; an edge that one triangle hides
+  from a whole receiver tile answers one query per cell) over the whole job, the L2
   flushed (256 MiB write) before every timed step, device time from CUDA
   events, max over ranks.
 * ``e2e``: the same steps with every radiomap and gradient copied back to

@@ -952,6 +952,7 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
         const int per = (min(jend - jb, width) + grp.warps - 1) / grp.warps;
         int next = jb + grp.rank * per;
         const int end = min(next + per, jend);
+        const int cells = __popc(__ballot_sync(kFull, active));  // a closed pair answers one query of each
         ShaftSearch q;
         Shaft sh;
         Ignore ig = ignore_none();
@@ -965,7 +966,6 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
                     const V3<float> near_end = edge_shaft(sc, list[jt], S, bounds, sh, ig);
                     q.start(sc, near_end, v3(0.5f * (bounds.lo[0] + bounds.hi[0]), 0.5f * (bounds.lo[1] + bounds.hi[1]),
                                              0.5f * (bounds.lo[2] + bounds.hi[2])));
-                    ++rays;
                 }
                 next += __popc(idle);
             } else if (idle == kFull) {
@@ -982,8 +982,10 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
                 bool closed = false;
                 if (q.leaf0 != 0) closed = q.test(sc, ig, sh);
                 else if (q.next != ShaftSearch::kNone) q.node(sc, stack);
-                if (closed) vis_words[tile * chunk + (jt - j0)] = 0u;
-                else if (q.done()) open_edges[atomicAdd(&num_open, 1)] = jt;
+                if (closed) {
+                    vis_words[tile * chunk + (jt - j0)] = 0u;
+                    rays += cells;
+                } else if (q.done()) open_edges[atomicAdd(&num_open, 1)] = jt;
                 if (closed || q.done()) jt = -1;
             }
         }

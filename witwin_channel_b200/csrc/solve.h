@@ -80,7 +80,7 @@ struct MainParams {
     unsigned long long* row_counter;
     int* status;
     unsigned long long* overflow_counter;
-    unsigned long long* ray_counter;  // segment/ray queries traced (optional)
+    unsigned long long* ray_counter;  // segment/ray queries answered (optional)
 };
 
 // Optional measurement of the main kernel: CUDA events bracket each launch
