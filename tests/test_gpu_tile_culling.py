@@ -4,8 +4,8 @@ that no receiver can have it (back projection outside a group's box, or one
 triangle across the whole shaft).  The same receivers in shuffled order fill
 their tiles with far-apart points, whose bounds span the scene and reject
 next to nothing, so both orders must give the same rows bit for bit.  The
-sizes take each number of warps per tile (8 below 1,024 tiles, 4 below 16,384,
-then 1), with ragged edges."""
+sizes take each number of warps per tile (8 below 1,024 tiles, 4 below 4,096,
+then 2; the UTD kernel 8, 4 and 2 from 4,096 and 16,384), with ragged edges."""
 
 from __future__ import annotations
 
@@ -40,7 +40,8 @@ def _rows(compiled, ep, mats, depth, rx_of):
     (1, 1, 12, 2, 2.0),        # one receiver
     (37, 29, 16, 3, 4.1),      # 8 warps per tile, ragged in both directions
     (189, 181, 40, 2, 1.9),    # 4 warps per tile
-    (733, 719, 9, 1, 0.21),    # 1 warp per tile
+    (403, 397, 12, 1, 0.5),    # 2 warps per tile, the UTD kernel 4
+    (733, 719, 9, 1, 0.21),    # 2 warps per tile in both
 ])
 def test_grid_rows_equal_shuffled_points(rows, cols, boxes, depth, spacing):
     layout = city_layout(boxes, 11)

@@ -8,19 +8,26 @@
 
 namespace wcb {
 
-// Warps per 32-cell tile of the reflection and diffraction kernels.  One warp
-// per tile keeps its batches full and waits for nobody, but its tiles take
-// unequal times, so it needs many waves to even out; eight warps share a tile
-// when tiles are few.  Measured (one B200, sum of the two kernels' calls): the
-// 1024^2 large city (32,768 tiles) 93 ms at 1, 105 at 4, 123 at 8; four
-// transmitters on 128^2 and 320^2 (2,048 and 12,800 tiles) 27.7 ms at 1, 22.4
-// at 4, 25.6 at 8; a 90 x 70 town (216 tiles) 7.3 ms at 1, 4.5 at 8.  FP64
-// keeps eight: its warps' sums are rounded to FP32 before they are added, so
-// another grouping would be another result.
+// Warps per 32-cell tile of the reflection and diffraction kernels.  Few warps
+// per tile keep their batches full and wait for nobody, but tiles take unequal
+// times, so they need many waves to even out; eight warps share a tile when
+// tiles are few.  Measured on one B200, ms of the kernels: reflection and
+// visibility of the 1024^2 large city (32,768 tiles) 23.5 + 55.1 at 1, 22.7 + 53.2
+// at 2; reflection of four transmitters on 128^2 and 320^2 (2,048 and 12,800
+// tiles) 5.89 at 4, 5.71 at 2 for the larger; a 90 x 70 town (216 tiles) 4.5 at 8,
+// 7.3 at 1 (whole call).  The UTD kernel, whose batches are dealt out evenly,
+// wants more: 0.34 at 4 and 0.25 at 8 on the canyon (2,048 tiles), the same at 1
+// and 2 on the city.  FP64 keeps eight: its warps' sums are rounded to FP32 before
+// they are added, so another grouping would be another result.
 template <typename T>
-static int tile_warps_for(long long tiles) {
+static int trace_tile_warps(long long tiles) {
     if (sizeof(T) == 8) return 8;
-    return tiles >= 16384 ? 1 : tiles >= 1024 ? 4 : 8;
+    return tiles >= 4096 ? 2 : tiles >= 1024 ? 4 : 8;
+}
+template <typename T>
+static int utd_tile_warps(long long tiles) {
+    if (sizeof(T) == 8) return 8;
+    return tiles >= 16384 ? 2 : tiles >= 4096 ? 4 : 8;
 }
 
 // LoS+transmission and diffraction go on `stream`, reflection on `side` (its
@@ -30,8 +37,9 @@ template <typename T, int NF>
 static void launch_nf(const MainParams& q0, unsigned blocks, int sdepth, size_t stack_bytes, cudaStream_t stream,
                cudaStream_t side, ComponentEvents* evs, const DiffractionPlan& dp) {
     const long long tiles = tiles_per_tx(q0) * q0.num_tx;
-    const int tw = tile_warps_for<T>(tiles);
+    const int tw = trace_tile_warps<T>(tiles), uw = utd_tile_warps<T>(tiles);
     const unsigned grid = unsigned((tiles * tw + kSplitWarps - 1) / kSplitWarps);
+    const unsigned utd_grid = unsigned((tiles * uw + kSplitWarps - 1) / kSplitWarps);
     const size_t split_stack = size_t(sdepth) * kSplitBlock * 4;
     const int c = q0.components;
     MainParams q = q0;
@@ -82,7 +90,7 @@ static void launch_nf(const MainParams& q0, unsigned blocks, int sdepth, size_t 
                     evs->vis.push_back(ev);
                 }
             }
-            k_diffract_utd<T, NF><<<grid, kSplitBlock, bytes, stream>>>(q, tw, j0, dp.chunk, dp.words,
+            k_diffract_utd<T, NF><<<utd_grid, kSplitBlock, bytes, stream>>>(q, uw, j0, dp.chunk, dp.words,
                                                                            static_cast<T*>(dp.carry));
             note_launch();
         }
