@@ -1044,6 +1044,12 @@ __global__ void __launch_bounds__(kSplitBlock, 2) k_diffract_utd(MainParams p, i
     const int warp = threadIdx.x >> 5;
     DiffShared<NF>* sh = reinterpret_cast<DiffShared<NF>*>(smem) + warp;
     float* red = reinterpret_cast<float*>(reinterpret_cast<DiffShared<NF>*>(smem) + kSplitWarps);
+    // the block's batch count, cleared before any group leaves: a block may hold
+    // tiles of two transmitters, and the first one's edges may end before this
+    // chunk while the second's do not
+    __shared__ int all_batches;
+    if (threadIdx.x == 0) all_batches = 0;
+    __syncthreads();
     const TileGroup grp = tile_group(tile_warps);
     const long long tile = grp.tile;
     int t = 0, r = 0;
@@ -1179,11 +1185,8 @@ __global__ void __launch_bounds__(kSplitBlock, 2) k_diffract_utd(MainParams p, i
     // straight code, and warps that drift apart in it flush each other's
     // instructions (no-instruction stalls 3.8 -> 0.5 per issue; one B200, before
     // and after: canyon 0.36 -> 0.32 ms, FP64 canyon 0.24 -> 0.16, four
-    // transmitters and frequencies 7.4 -> 5.7).  Groups without a tile have left
-    // the block, which the barrier allows.
-    __shared__ int all_batches;
-    if (threadIdx.x == 0) all_batches = 0;
-    __syncthreads();
+    // transmitters and frequencies 7.4 -> 5.7).  Groups without a tile or without
+    // edges in this chunk have left the block, which the barrier allows.
     if (lane == 0) atomicMax(&all_batches, (hi - lo + 31) / 32);
     __syncthreads();
     const int batches = all_batches;
