@@ -385,6 +385,15 @@ int wcb_cfr(const int32_t* tx_id, const int32_t* rx_id, const float* delay_s, co
             const double* frequencies, int32_t normalize_delays, float* out, void* workspace,
             int64_t workspace_bytes, void* stream);
 
+/* wcb_cfr behind a check that the host has not read yet: `refuse` (device
+ * byte, or NULL) is tested when the kernels start, and when it is not zero
+ * they write no output and walk no records.  A table out of canonical order is
+ * refused this way: its links' record ranges span foreign records. */
+int wcb_cfr_guarded(const int32_t* tx_id, const int32_t* rx_id, const float* delay_s, const float* path_field,
+                    int64_t num_paths, int32_t num_tx, int32_t num_rx, int32_t num_freq, double f0, double df,
+                    const double* frequencies, int32_t normalize_delays, const uint8_t* refuse, float* out,
+                    void* workspace, int64_t workspace_bytes, void* stream);
+
 /* Standalone field operators (reference kernels/fields.py facades).  All
  * arrays are device f32; complex outputs interleaved.  N rows. */
 int wcb_field_free_space(int64_t n, const float* source, const float* target, const float* tx_power,

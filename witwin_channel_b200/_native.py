@@ -206,6 +206,7 @@ EXPORTED_SYMBOLS = (
     "wcb_rows_decode",
     "wcb_cfr_workspace_size",
     "wcb_cfr",
+    "wcb_cfr_guarded",
     "wcb_field_free_space",
     "wcb_field_reflection_sequence",
     "wcb_field_transmission_sequence",
@@ -286,6 +287,7 @@ def load() -> ctypes.CDLL:
     lib.wcb_cfr_workspace_size.argtypes = [ctypes.c_int32, ctypes.c_int32, _i64p]
     lib.wcb_cfr.argtypes = [_vp, _vp, _vp, _vp, ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                             ctypes.c_double, ctypes.c_double, _vp, ctypes.c_int32, _vp, _vp, ctypes.c_int64, _vp]
+    lib.wcb_cfr_guarded.argtypes = lib.wcb_cfr.argtypes[:12] + [_vp] + lib.wcb_cfr.argtypes[12:]
     lib.wcb_field_free_space.argtypes = [ctypes.c_int64] + [_vp] * 5 + [ctypes.c_double] + [_vp] * 7 + [_vp]
     lib.wcb_field_reflection_sequence.argtypes = [ctypes.c_int64, ctypes.c_int32] + [_vp] * 12 + [ctypes.c_double] + [_vp] * 7 + [_vp]
     lib.wcb_field_transmission_sequence.argtypes = [ctypes.c_int64, ctypes.c_int32] + [_vp] * 8 + [

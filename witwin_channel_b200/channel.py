@@ -18,6 +18,7 @@ import torch
 from . import _native, engine
 
 _CFR_WORKSPACE = engine.Workspace()
+_UNORDERED = "paths must be in the canonical (rx, tx) order of an exported path table"
 
 
 def _coefficients(paths) -> torch.Tensor:
@@ -47,15 +48,19 @@ def cfr(paths, frequencies, *, num_tx: int, num_rx: int, normalize_delays: bool 
     # waits for the work queued before it)
     freqs = frequencies.to(device=device, dtype=torch.float64).contiguous() if df == 0.0 else None
     n = int(paths.tx_id.shape[0])
+    refuse = checked = None
     if n > 1:
-        # checked on the device; read below, after the spectrum's launch, so the
-        # host does not wait with an idle device (an unordered table's spectrum
-        # stays within its buffers and is dropped)
         key = paths.rx_id.long() * max(int(num_tx), 1) + paths.tx_id.long()
-        unordered = torch.empty((), dtype=torch.bool, pin_memory=True)
-        unordered.copy_((key[1:] < key[:-1]).any(), non_blocking=True)
-        checked = torch.cuda.Event()
-        checked.record()
+        refuse = (key[1:] < key[:-1]).any()
+        if device.type == "cuda":
+            # read below, after the spectrum's launch, so the host does not wait with
+            # an idle device; the kernels test it first and leave at once
+            unordered = torch.empty((), dtype=torch.bool, pin_memory=True)
+            unordered.copy_(refuse, non_blocking=True)
+            checked = torch.cuda.Event()
+            checked.record()
+        elif bool(refuse):
+            raise ValueError(_UNORDERED)
     out = torch.empty((num_tx, num_rx, K), dtype=torch.complex64, device=device)
     a = _coefficients(paths).contiguous()
     lib = _native.load()
@@ -63,18 +68,18 @@ def cfr(paths, frequencies, *, num_tx: int, num_rx: int, normalize_delays: bool 
     _native.check(lib.wcb_cfr_workspace_size(int(num_tx), int(num_rx), ctypes.byref(nbytes)), "wcb_cfr_workspace_size")
     ws = _CFR_WORKSPACE.get(nbytes.value, device)
     _native.check(
-        lib.wcb_cfr(_native.ptr(paths.tx_id.contiguous()) if n else None,
-                    _native.ptr(paths.rx_id.contiguous()) if n else None,
-                    _native.ptr(paths.delay_s.float().contiguous()) if n else None,
-                    _native.ptr(torch.view_as_real(a)) if n else None, n, int(num_tx), int(num_rx), K,
-                    float(f_host[0]), df, _native.ptr(freqs), int(bool(normalize_delays)), _native.ptr(out),
-                    _native.ptr(ws), ws.numel(), _native.stream_handle(device)),
-        "wcb_cfr",
+        lib.wcb_cfr_guarded(_native.ptr(paths.tx_id.contiguous()) if n else None,
+                            _native.ptr(paths.rx_id.contiguous()) if n else None,
+                            _native.ptr(paths.delay_s.float().contiguous()) if n else None,
+                            _native.ptr(torch.view_as_real(a)) if n else None, n, int(num_tx), int(num_rx), K,
+                            float(f_host[0]), df, _native.ptr(freqs), int(bool(normalize_delays)), _native.ptr(refuse),
+                            _native.ptr(out), _native.ptr(ws), ws.numel(), _native.stream_handle(device)),
+        "wcb_cfr_guarded",
     )
-    if n > 1:
+    if checked is not None:
         checked.synchronize()
         if bool(unordered):
-            raise ValueError("paths must be in the canonical (rx, tx) order of an exported path table")
+            raise ValueError(_UNORDERED)
     return out
 
 

@@ -35,7 +35,10 @@ struct CfrParams {
     double f0, df;            // uniform grid (df != 0)
     const double* freqs;      // explicit grid (df == 0)
     int normalize;
+    const unsigned char* refuse;  // device byte, or null: not zero = leave the outputs alone
     float* out;               // (T,R,NF) complex
+
+    WCB_D bool refused() const { return refuse != nullptr && *refuse != 0; }
 };
 
 // reduce 2 pi x (cycles) to [-pi, pi] in FP64 and return cos/sin in FP32; the
@@ -49,10 +52,12 @@ WCB_D void cycles_sincos(double cycles, float* s, float* c) {
 // [start, end) record range of every link from one pass over the canonical
 // records (each link's records are contiguous); links without records keep
 // the empty range the caller cleared to zero.
-__global__ void k_link_ranges(long long n, const int* tx, const int* rx, int num_rx, int* start, int* end) {
+__global__ void k_link_ranges(CfrParams p, int* start, int* end) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const long long cell = (long long)tx[i] * num_rx + rx[i];
+    const long long n = p.count;
+    if (i >= n || p.refused()) return;
+    const int *tx = p.tx, *rx = p.rx;
+    const long long cell = (long long)tx[i] * p.num_rx + rx[i];
     if (i == 0 || tx[i - 1] != tx[i] || rx[i - 1] != rx[i]) start[cell] = int(i);
     if (i == n - 1 || tx[i + 1] != tx[i] || rx[i + 1] != rx[i]) end[cell] = int(i + 1);
 }
@@ -71,7 +76,7 @@ __global__ void __launch_bounds__(kCfrWarps * 32) k_cfr(CfrParams p, const int* 
     const int L = threadIdx.x & (kLinkLanes - 1);
     const int lane = threadIdx.x & 31;
     const long long cells = (long long)p.num_tx * p.num_rx;
-    if (cell >= cells) return;  // both warps of a link leave together
+    if (cell >= cells || p.refused()) return;  // both warps of a link leave together
     const int beg = link_start[cell], end = link_end[cell];
     double tau0 = 0.0;
     if (p.normalize && end > beg) {
@@ -137,7 +142,7 @@ __global__ void __launch_bounds__(kCfrWarps * 32) k_cfr_pairs(CfrParams p, const
     const int L = threadIdx.x & (kLinkLanes - 1);
     const int lane = threadIdx.x & 31;
     const long long cells = (long long)p.num_tx * p.num_rx;
-    if (cell >= cells) return;  // both warps of a link leave together
+    if (cell >= cells || p.refused()) return;  // both warps of a link leave together
     const int beg = link_start[cell], end = link_end[cell];
     double tau0 = 0.0;
     if (p.normalize && end > beg) {
@@ -194,10 +199,11 @@ extern "C" int wcb_cfr_workspace_size(int32_t num_tx, int32_t num_rx, int64_t* b
     return WCB_OK;
 }
 
-extern "C" int wcb_cfr(const int32_t* tx_id, const int32_t* rx_id, const float* delay_s, const float* path_field,
-                       int64_t num_paths, int32_t num_tx, int32_t num_rx, int32_t num_freq, double f0, double df,
-                       const double* frequencies, int32_t normalize_delays, float* out, void* workspace,
-                       int64_t workspace_bytes, void* stream) {
+extern "C" int wcb_cfr_guarded(const int32_t* tx_id, const int32_t* rx_id, const float* delay_s,
+                               const float* path_field, int64_t num_paths, int32_t num_tx, int32_t num_rx,
+                               int32_t num_freq, double f0, double df, const double* frequencies,
+                               int32_t normalize_delays, const uint8_t* refuse, float* out, void* workspace,
+                               int64_t workspace_bytes, void* stream) {
     if (num_paths < 0 || num_paths > INT_MAX || num_tx < 0 || num_rx < 0 || out == nullptr)
         return WCB_ERR_INVALID_ARGUMENT;
     if (num_freq < 1) return WCB_ERR_INVALID_ARGUMENT;
@@ -213,11 +219,6 @@ extern "C" int wcb_cfr(const int32_t* tx_id, const int32_t* rx_id, const float* 
     int* link_end = link_start + need / 8;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaMemsetAsync(workspace, 0, size_t(need), s);
-    if (num_paths > 0) {
-        wcb::k_link_ranges<<<unsigned((num_paths + 255) / 256), 256, 0, s>>>(num_paths, tx_id, rx_id, num_rx,
-                                                                            link_start, link_end);
-        wcb::note_launch();
-    }
     wcb::CfrParams p;
     p.tx = tx_id;
     p.rx = rx_id;
@@ -231,7 +232,12 @@ extern "C" int wcb_cfr(const int32_t* tx_id, const int32_t* rx_id, const float* 
     p.df = df;
     p.freqs = frequencies;
     p.normalize = normalize_delays != 0;
+    p.refuse = refuse;
     p.out = out;
+    if (num_paths > 0) {
+        wcb::k_link_ranges<<<unsigned((num_paths + 255) / 256), 256, 0, s>>>(p, link_start, link_end);
+        wcb::note_launch();
+    }
     const unsigned blocks = unsigned((cells + wcb::kLinksPerBlock - 1) / wcb::kLinksPerBlock);
     const unsigned th = wcb::kCfrWarps * 32;
     const int per_lane = (num_freq + wcb::kLinkLanes - 1) / wcb::kLinkLanes;
@@ -252,4 +258,12 @@ extern "C" int wcb_cfr(const int32_t* tx_id, const int32_t* rx_id, const float* 
 #undef WCB_CFR_LAUNCH
     wcb::note_launch();
     return cudaGetLastError() == cudaSuccess ? WCB_OK : WCB_ERR_CUDA;
+}
+
+extern "C" int wcb_cfr(const int32_t* tx_id, const int32_t* rx_id, const float* delay_s, const float* path_field,
+                       int64_t num_paths, int32_t num_tx, int32_t num_rx, int32_t num_freq, double f0, double df,
+                       const double* frequencies, int32_t normalize_delays, float* out, void* workspace,
+                       int64_t workspace_bytes, void* stream) {
+    return wcb_cfr_guarded(tx_id, rx_id, delay_s, path_field, num_paths, num_tx, num_rx, num_freq, f0, df, frequencies,
+                           normalize_delays, nullptr, out, workspace, workspace_bytes, stream);
 }
