@@ -60,3 +60,20 @@ def test_permuted_table_is_refused(stream):
         t = _table(order)
         with pytest.raises(ValueError, match="canonical"):
             cfr(t, np.arange(300) * 1e5, num_tx=1, num_rx=LINKS)
+
+
+def test_check_is_read_after_its_own_copy(monkeypatch):
+    """The event that the host waits for is recorded on the stream that holds
+    the check's copy: the table's device, whatever the current device is."""
+    streams = []
+
+    class Event(torch.cuda.Event):
+        def record(self, stream=None):
+            streams.append(stream)
+            super().record(stream)
+
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    t = _table(torch.arange(LINKS * PER_LINK))
+    cfr(t, np.arange(300) * 1e5, num_tx=1, num_rx=LINKS)
+    assert [s.cuda_stream for s in streams] == [_native.stream_handle(t.rx_id.device)]
+    assert streams[0].device == t.rx_id.device

@@ -58,7 +58,7 @@ def cfr(paths, frequencies, *, num_tx: int, num_rx: int, normalize_delays: bool 
             unordered = torch.empty((), dtype=torch.bool, pin_memory=True)
             unordered.copy_(refuse, non_blocking=True)
             checked = torch.cuda.Event()
-            checked.record()
+            checked.record(torch.cuda.current_stream(device))
         elif bool(refuse):
             raise ValueError(_UNORDERED)
     out = torch.empty((num_tx, num_rx, K), dtype=torch.complex64, device=device)
