@@ -116,6 +116,15 @@ WCB_HD_OOL FresnelPair<T> fresnel_pos(T x) {
     FresnelPair<T> out;
     const T z = x * T(1.2533141373155002512);  // sqrt(pi/2)
     const T y = z * z;
+    if (sizeof(T) == 4 && y > T(1e8)) {
+        // h = (1/(2 y^2) + j/y)/2 to within 4 / y^2 relative: the FP32 sums' common
+        // denominators grow as y^4 and overflow from y = 4.3e9 (x = 5.2e4)
+        const T r = T(1) / y;
+        out.h = cx(T(0.25) * r * r, T(0.5) * r);
+        out.has_pole = false;
+        out.pole = cx(T(0), T(0));
+        return out;
+    }
     T s0, s1;
     Trapezium<T>::sums(y, &s0, &s1);
     out.h = cx(T(0.5) * s1, T(0.5) * y * s0);
