@@ -870,9 +870,12 @@ WCB_D V3<float> edge_shaft(const SceneDev& sc, int edge, V3<double> S, const Til
     const float tw = fabsf(e.x) * half.x + fabsf(e.y) * half.y + fabsf(e.z) * half.z;
     const float rw = length(half);
     const float size = fmaxf(norm1(mid) + norm1(half), norm1(c) + hl);
-    const float slack = 1e-3f + 2e-5f * (size + rs);
+    // FP32 forms ts and rs within a few 2^-24 of the transmitter's distance; rs is
+    // widened by that, which counts for a transmitter close to the edge's axis
+    const float slack = 1e-3f + 2e-5f * (size + rs + fabsf(ts));
+    const float rs_lo = fmaxf(rs - 1e-6f * (rs + fabsf(ts)), 0.f), rs_hi = rs + 1e-6f * (rs + fabsf(ts));
     const float r_lo = fmaxf(rm - rw - slack, 0.f), r_hi = rm + rw + slack;
-    const float w_lo = rs / fmaxf(rs + r_hi, 1e-6f), w_hi = rs / fmaxf(rs + r_lo, 1e-6f);
+    const float w_lo = rs_lo / (rs_lo + r_hi), w_hi = rs_hi / fmaxf(rs_hi + r_lo, 1e-30f);
     const float d_lo = tm - tw - ts, d_hi = tm + tw - ts;
     const float t_lo = ts + fminf(d_lo * w_lo, d_lo * w_hi) - slack, t_hi = ts + fmaxf(d_hi * w_lo, d_hi * w_hi) + slack;
     const float q_lo = fminf(fmaxf(t_lo, -hl), hl), q_hi = fminf(fmaxf(t_hi, -hl), hl);
