@@ -203,10 +203,13 @@ def _layout(values: torch.Tensor, rx: dict) -> torch.Tensor:
     return values.contiguous()
 
 
-def _layout_slots(values: torch.Tensor, rx: dict) -> torch.Tensor:
-    """:func:`_layout` of every slot of ``values`` (slots, T, R)."""
-    flat = _layout(values.reshape(values.shape[0] * values.shape[1], values.shape[2]), rx)
-    return flat.reshape(values.shape[0], values.shape[1], *flat.shape[1:])
+def _layout_slots(values: torch.Tensor, rx: dict) -> tuple[torch.Tensor, ...]:
+    """:func:`_layout` of every slot of ``values`` (slots, T, R), each grid map
+    with a storage of its own (keeping or saving one keeps no other)."""
+    if rx["kind"] == "grid":
+        rows, cols = rx["shape"]
+        return torch.unbind_copy(values.reshape(*values.shape[:2], rows, cols).transpose(2, 3))
+    return values.unbind(0)
 
 
 def _metadata(config: Config, counts: dict, path_count: int, launches: int, extra: dict) -> dict:
@@ -309,10 +312,12 @@ def solve(scene: Any, config: Config, *, reference_frequency_hz, precision: str 
     field = cells.field[0]
     extra_components = tuple(n for n in _OPTIONAL_COMPONENTS if n in config.components)
     names = _BASE_COMPONENTS + extra_components
-    # the named slots are the first ones: laid out in one launch each for powers and fields
-    comp_power = dict(zip(names, _layout_slots(cells.comp_power[:len(names), 0], rx).unbind(0)))
-    comp_fields = dict(zip(names, _layout_slots(cells.comp_field[:len(names), 0], rx).unbind(0))) \
-        if config.return_field else {n: torch.empty((0,), dtype=torch.complex64, device=device) for n in names}
+    slots = 1 + max(_SLOTS[n] for n in names)
+    power_maps = _layout_slots(cells.comp_power[:slots, 0], rx)
+    comp_power = {n: power_maps[_SLOTS[n]] for n in names}
+    field_maps = _layout_slots(cells.comp_field[:slots, 0], rx) if config.return_field else None
+    comp_fields = {n: field_maps[_SLOTS[n]] if config.return_field
+                   else torch.empty((0,), dtype=torch.complex64, device=device) for n in names}
     exact = None
     if "diffraction" in config.components and rx["kind"] == "grid" and len(scene.receivers) == 1:
         exact = _layout(cells.diff_vec_power[0], rx)
