@@ -14,7 +14,8 @@ synthetic (seeded); no dataset is read.
   discovery bounces of every solve in the step; an edge that one triangle hides
   from a whole receiver tile answers one query per cell) over the whole job, the L2
   flushed (256 MiB write) before every timed step, device time from CUDA
-  events, max over ranks.
+  events, max over ranks.  ``rays_traced_per_s`` counts what was traced for
+  those queries: segments, and one search per (tile, edge) pair.
 * ``e2e``: the same steps with every radiomap and gradient copied back to
   host memory, timed by the host clock.
 * ``roofline``: the step's dominant kernel by serialised time (the
@@ -271,6 +272,7 @@ def run_native(args) -> None:
     prof = _native.profile_read()
     _native.profile_enable(False)
     rays_per_step = float(prof["acc_rays"])
+    traced_per_step = float(prof["acc_rays_traced"])
     vjp_ms, vjp_records, vjp_launches = (prof["acc_vjp_diffraction_ms"], prof["acc_vjp_diffraction_records"],
                                          prof["acc_vjp_diffraction_launches"])
     if world > 1:
@@ -311,11 +313,11 @@ def run_native(args) -> None:
         t = torch.tensor([step_ms, e2e_ms], dtype=torch.float64, device=device)
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         step_ms_all, e2e_ms_all = float(t[0]), float(t[1])
-        r = torch.tensor([rays_per_step], dtype=torch.float64, device=device)
+        r = torch.tensor([rays_per_step, traced_per_step], dtype=torch.float64, device=device)
         dist.all_reduce(r, op=dist.ReduceOp.SUM)
-        rays_all = float(r[0])
+        rays_all, traced_all = float(r[0]), float(r[1])
     else:
-        step_ms_all, e2e_ms_all, rays_all = step_ms, e2e_ms, rays_per_step
+        step_ms_all, e2e_ms_all, rays_all, traced_all = step_ms, e2e_ms, rays_per_step, traced_per_step
     value = rays_all * args.steps / (step_ms_all / 1000.0)
     e2e_value = rays_all * e2e_steps / (e2e_ms_all / 1000.0)
     single = world == 1
@@ -373,6 +375,8 @@ def run_native(args) -> None:
                 "frequencies_hz": list(BATCH_FREQS),
                 "max_depth": 3,
                 "rays_per_step": rays_all,
+                "rays_traced_per_step": traced_all,
+                "rays_traced_per_s": traced_all * args.steps / (step_ms_all / 1000.0),
                 "per_step_ms": [round(x, 3) for x in per_step],
                 "l2": "flushed (256 MiB write) before every timed step",
                 "parallelism": (f"{world} ranks: the 32 (scene, Tx) jobs partitioned (longest processing time first), "
@@ -433,8 +437,10 @@ def _canyon_run(args, device, steps: int = 50) -> dict:
     ends = [torch.cuda.Event(enable_timing=True) for _ in range(steps)]
     rays = 0
     main_rays = 0
+    traced = 0
     kernel_ms: dict[str, float] = {}
     kernel_rays: dict[str, int] = {}
+    kernel_traced: dict[str, int] = {}
     last_prof: dict = {}
     torch.cuda.synchronize()
     for i in range(steps):
@@ -445,10 +451,13 @@ def _canyon_run(args, device, steps: int = 50) -> dict:
         prof = _native.profile_read()
         rays += prof["rays"] + prof["prep_rays"]
         main_rays += prof["rays"]
+        traced += prof["rays_traced"] + prof["prep_rays"]
         for k, v in prof["kernel_ms"].items():
             kernel_ms[k] = kernel_ms.get(k, 0.0) + v
         for k, v in prof["kernel_rays"].items():
             kernel_rays[k] = kernel_rays.get(k, 0) + v
+        for k, v in prof["kernel_rays_traced"].items():
+            kernel_traced[k] = kernel_traced.get(k, 0) + v
         last_prof = prof
     torch.cuda.synchronize()
     _native.profile_enable(False)
@@ -472,7 +481,7 @@ def _canyon_run(args, device, steps: int = 50) -> dict:
     torch.cuda.synchronize()
     e2e_ms = e0.elapsed_time(e1)
     e2e_value = rays / (e2e_ms / 1000.0)
-    # dominant per-cell kernel: its rays and the bytes it writes per cell (slot
+    # dominant per-cell kernel: the rays it traces and the bytes it writes per cell (slot
     # values; for diffraction one visibility bit per kept edge)
     peaks = _peaks()
     hbm = float(peaks.get("hbm_gbs", HBM_FALLBACK))
@@ -483,7 +492,7 @@ def _canyon_run(args, device, steps: int = 50) -> dict:
     cell_bytes = {"k_reflect": 12, "k_diffract_vis": edges_kept / 8, "k_diffract_utd": 16 + edges_kept / 8,
                   "k_los_trans": 12}[dominant]
     rays_of = {"k_reflect": "k_reflect", "k_diffract_vis": "k_diffract", "k_los_trans": "k_los_trans"}
-    dom_rays = kernel_rays.get(rays_of.get(dominant, ""), 0)
+    dom_rays = kernel_traced.get(rays_of.get(dominant, ""), 0)
     bytes_per_launch = dom_rays / steps * _bytes_per_ray(faces) + cells_n * cell_bytes
     launch_ms = kernel_ms.get(dominant, 0.0) / steps
     achieved = bytes_per_launch / (launch_ms / 1000.0) / 1e9 if launch_ms > 0 else 0.0
@@ -497,9 +506,12 @@ def _canyon_run(args, device, steps: int = 50) -> dict:
         "steps": steps,
         "triangles": faces,
         "rays_per_step": rays / steps,
+        "rays_traced_per_step": traced / steps,
+        "rays_traced_per_s": traced / (step_ms / 1000.0),
         "per_cell_kernel_rays_per_step": main_rays / steps,
         "kernel_ms_per_step": {k: v / steps for k, v in kernel_ms.items()},
         "kernel_rays_per_step": {k: v / steps for k, v in kernel_rays.items()},
+        "kernel_rays_traced_per_step": {k: v / steps for k, v in kernel_traced.items()},
         "reflection_candidates_per_depth": last_prof.get("chains"),
         "diffraction_edges_after_prefilter": last_prof.get("edges"),
         "cells_per_step": cells_n,
@@ -805,6 +817,7 @@ def _large_run(device, steps: int = 2) -> dict:
         "solve_ms": e[0].elapsed_time(e[1]) / steps,
         "kernel_ms": prof["kernel_ms"],
         "rays": rays,
+        "rays_traced": prof["rays_traced"] + prof["prep_rays"],
         "rays_per_s_kernels": rays / ((prof["main_ms"] + prof["prep_ms"]) / 1000.0),
         "paths": int(res.metadata["counts"]["path_count"]),
         "cfr_ms": cfr_ms,

@@ -518,7 +518,9 @@ int wcb_rows_replay(const wcb_scene* scene, const wcb_frozen_rows* rows, const w
 
 /* Measurement: when enabled, wcb_solve brackets its candidate preparation and
  * its main kernel with CUDA events on the solve stream and counts the rays
- * (segment visibility / penetration queries) the main kernel traces.
+ * (segment visibility / penetration queries) the main kernel answers: one per
+ * traced segment, and one per cell where one triangle hides an edge from a
+ * whole tile of cells.  wcb_profile_read_traced gives what was traced for them.
  * wcb_profile_read returns the last solve's figures: values[0] main-kernel ms,
  * values[1] preparation ms, values[2] main-kernel rays, values[3] main-kernel
  * launches, values[4] preparation rays (discovery bounces, edge prefilter),
@@ -534,6 +536,14 @@ int wcb_rows_replay(const wcb_scene* scene, const wcb_frozen_rows* rows, const w
  * `values` holds 23 doubles. */
 int wcb_profile_enable(int32_t enabled);
 int wcb_profile_read(double* values);
+
+/* The rays traced for the queries that wcb_profile_read counts: segments, and
+ * one search per (tile, edge) pair in place of the queries of a hidden pair's
+ * cells.  values[0] main-kernel rays of the last solve (beside values[2] of
+ * wcb_profile_read), values[1] those of the diffraction kernels (beside
+ * values[11]), values[2] accumulated over every solve, preparation included
+ * (beside values[19]).  `values` holds 3 doubles. */
+int wcb_profile_read_traced(double* values);
 
 /* Runtime info: writes a NUL-terminated description (architecture, build). */
 int wcb_build_info(char* buffer, int64_t capacity);

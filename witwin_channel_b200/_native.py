@@ -215,6 +215,7 @@ EXPORTED_SYMBOLS = (
     "wcb_rows_replay",
     "wcb_profile_enable",
     "wcb_profile_read",
+    "wcb_profile_read_traced",
     "wcb_build_info",
     "wcb_launch_count",
 )
@@ -300,6 +301,7 @@ def load() -> ctypes.CDLL:
                                     ctypes.c_int32, ctypes.c_int32, ctypes.POINTER(ReplayOutputs), _vp, _vp]
     lib.wcb_profile_enable.argtypes = [ctypes.c_int32]
     lib.wcb_profile_read.argtypes = [ctypes.POINTER(ctypes.c_double)]
+    lib.wcb_profile_read_traced.argtypes = [ctypes.POINTER(ctypes.c_double)]
     lib.wcb_build_info.argtypes = [ctypes.c_char_p, ctypes.c_int64]
     lib.wcb_launch_count.restype = ctypes.c_int64
     for name in EXPORTED_SYMBOLS:
@@ -351,11 +353,16 @@ def profile_enable(enabled: bool) -> None:
 def profile_read() -> dict:
     vals = (ctypes.c_double * 23)()
     check(load().wcb_profile_read(vals), "wcb_profile_read")
+    traced = (ctypes.c_double * 3)()
+    check(load().wcb_profile_read_traced(traced), "wcb_profile_read_traced")
     return {"main_ms": vals[0], "prep_ms": vals[1], "rays": int(vals[2]), "main_launches": int(vals[3]),
             "prep_rays": int(vals[4]),
             "kernel_ms": {"k_los_trans": vals[5], "k_reflect": vals[6], "k_diffract": vals[7], "k_finalize": vals[8],
                           "k_diffract_vis": vals[18], "k_diffract_utd": vals[7] - vals[18]},
             "kernel_rays": {"k_los_trans": int(vals[9]), "k_reflect": int(vals[10]), "k_diffract": int(vals[11])},
+            "rays_traced": int(traced[0]), "acc_rays_traced": int(traced[2]),
+            "kernel_rays_traced": {"k_los_trans": int(vals[9]), "k_reflect": int(vals[10]),
+                                   "k_diffract": int(traced[1])},
             "chains": [int(v) for v in vals[12:17]], "edges": int(vals[17]),
             "acc_rays": int(vals[19]), "acc_vjp_diffraction_ms": vals[20],
             "acc_vjp_diffraction_records": int(vals[21]), "acc_vjp_diffraction_launches": int(vals[22])}

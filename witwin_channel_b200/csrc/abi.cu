@@ -252,7 +252,7 @@ int wcb_profile_enable(int32_t enabled) {
     wcb::ProfileState& st = wcb::profile_state();
     st.enabled = enabled != 0;
     if (st.enabled) {
-        st.acc_rays = 0;
+        st.acc_rays = st.acc_rays_traced = 0;
         st.acc_vjp_diff_ms = 0.0;
         st.acc_vjp_diff_records = 0;
         st.acc_vjp_diff_launches = 0;
@@ -277,6 +277,15 @@ int wcb_profile_read(double* values) {
     values[20] = st.acc_vjp_diff_ms;
     values[21] = double(st.acc_vjp_diff_records);
     values[22] = double(st.acc_vjp_diff_launches);
+    return WCB_OK;
+}
+
+int wcb_profile_read_traced(double* values) {
+    if (values == nullptr) return WCB_ERR_INVALID_ARGUMENT;
+    const wcb::ProfileState& st = wcb::profile_state();
+    values[0] = double(st.rays_traced);
+    values[1] = double(st.diffract_traced);
+    values[2] = double(st.acc_rays_traced);
     return WCB_OK;
 }
 

@@ -626,7 +626,7 @@ int solve(const SceneHandle* h, const wcb_solve_desc* d, const wcb_materials* m,
     int* edge_count = reinterpret_cast<int*>(base + L.edge_count);
     unsigned long long* overflow = reinterpret_cast<unsigned long long*>(base + L.overflow);
     unsigned long long* ray_counter = overflow + 1;       // preparation rays (discovery, edge prefilter)
-    unsigned long long* main_ray_counter = overflow + 2;  // per-cell kernel rays: los+trans, reflection, diffraction
+    unsigned long long* main_ray_counter = overflow + 2;  // per-cell kernel rays: los+trans, reflection, diffraction (3)
     const bool fp64 = d->precision == 1;
     ProfileState& prof = profile_state();
     cudaEvent_t ev_prep = nullptr, ev_main0 = nullptr, ev_main1 = nullptr;
@@ -636,7 +636,7 @@ int solve(const SceneHandle* h, const wcb_solve_desc* d, const wcb_materials* m,
         cudaEventCreate(&ev_main1);
         cudaEventRecord(ev_prep, stream);
         prof.main_ms = prof.prep_ms = 0.0;
-        prof.rays = 0;
+        prof.rays = prof.rays_traced = 0;
         prof.prep_rays = 0;
         prof.main_launches = 0;
     }
@@ -922,8 +922,8 @@ int solve(const SceneHandle* h, const wcb_solve_desc* d, const wcb_materials* m,
     }
     if (prof.enabled) {
         cudaEventRecord(ev_main1, stream);
-        unsigned long long nr[4] = {0, 0, 0, 0};
-        cudaMemcpyAsync(nr, ray_counter, 32, cudaMemcpyDeviceToHost, stream);
+        unsigned long long nr[6] = {0, 0, 0, 0, 0, 0};
+        cudaMemcpyAsync(nr, ray_counter, sizeof(nr), cudaMemcpyDeviceToHost, stream);
         int cc[kMaxDepth] = {0, 0, 0, 0, 0};
         int ec = 0;
         cudaMemcpyAsync(cc, chain_counts, sizeof(cc), cudaMemcpyDeviceToHost, stream);
@@ -936,9 +936,13 @@ int solve(const SceneHandle* h, const wcb_solve_desc* d, const wcb_materials* m,
         prof.prep_ms = a;
         prof.main_ms = b;
         prof.prep_rays = (long long)nr[0];
-        prof.rays = (long long)(nr[1] + nr[2] + nr[3]);
+        prof.rays = (long long)(nr[1] + nr[2] + nr[3] + nr[4]);
+        prof.rays_traced = (long long)(nr[1] + nr[2] + nr[3] + nr[5]);
         prof.acc_rays += prof.rays + prof.prep_rays;
+        prof.acc_rays_traced += prof.rays_traced + prof.prep_rays;
         for (int i = 0; i < 3; ++i) prof.kernel_rays[i] = (long long)nr[1 + i];
+        prof.kernel_rays[2] += (long long)nr[4];
+        prof.diffract_traced = (long long)(nr[3] + nr[5]);
         for (int i = 0; i < 4; ++i) prof.kernel_ms[i] = comp_ms[i];
         prof.diffract_vis_ms = vis_ms;
         for (int i = 0; i < kMaxDepth; ++i) prof.chains[i] = cc[i];

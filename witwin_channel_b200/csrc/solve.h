@@ -80,7 +80,10 @@ struct MainParams {
     unsigned long long* row_counter;
     int* status;
     unsigned long long* overflow_counter;
-    unsigned long long* ray_counter;  // segment/ray queries answered (optional)
+    // segment/ray queries traced (optional); the diffraction visibility kernel's is
+    // followed by the queries that a closed (tile, edge) pair answers for its cells
+    // and by the shaft searches that closed or opened the pairs
+    unsigned long long* ray_counter;
 };
 
 // Optional measurement of the main kernel: CUDA events bracket each launch
@@ -89,16 +92,19 @@ struct ProfileState {
     bool enabled = false;
     double main_ms = 0.0;        // summed time of the per-cell kernels of the last solve
     double prep_ms = 0.0;        // candidate preparation time of the last solve
-    long long rays = 0;          // rays traced by the per-cell kernels in the last solve
+    long long rays = 0;          // queries answered by the per-cell kernels in the last solve
+    long long rays_traced = 0;   // rays that they traced for it (segments and shaft searches)
     long long prep_rays = 0;     // rays traced while preparing candidates (discovery, edge prefilter)
     long long main_launches = 0;
     double kernel_ms[4] = {0, 0, 0, 0};       // los+transmission, reflection, diffraction, finalize
     double diffract_vis_ms = 0.0;             // the visibility part of the diffraction time
-    long long kernel_rays[3] = {0, 0, 0};     // los+transmission, reflection, diffraction
+    long long kernel_rays[3] = {0, 0, 0};     // queries of los+transmission, reflection, diffraction
+    long long diffract_traced = 0;            // rays traced for the diffraction queries
     long long chains[5] = {0, 0, 0, 0, 0};    // reflection candidates per depth (first transmitter)
     long long edges = 0;                      // diffraction edges kept by the prefilter (first transmitter)
     // accumulated since profiling was last enabled (over every solve and VJP)
-    long long acc_rays = 0;                   // rays traced by all solves (preparation and per-cell kernels)
+    long long acc_rays = 0;                   // queries of all solves (preparation and per-cell kernels)
+    long long acc_rays_traced = 0;            // rays traced for them
     double acc_vjp_diff_ms = 0.0;             // reverse-mode diffraction VJP kernel time
     long long acc_vjp_diff_records = 0;       // diffraction records it processed
     long long acc_vjp_diff_launches = 0;
