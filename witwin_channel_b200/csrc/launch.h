@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <utility>
 #include <vector>
 
@@ -17,6 +18,18 @@ struct ComponentEvents {
     cudaEvent_t end[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> vis;  // around each diffraction visibility launch
 };
+
+// Raises a kernel's dynamic shared memory limit to `bytes`, once per device: the
+// attribute belongs to the device that is current when it is set.  `done` holds
+// a bit per device.
+inline void raise_shared_limit(const void* kernel, int bytes, std::atomic<unsigned long long>& done) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return;
+    const unsigned long long bit = 1ull << (device & 63);
+    if (done.load(std::memory_order_acquire) & bit) return;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+        done.fetch_or(bit, std::memory_order_release);
+}
 
 struct DiffractionPlan {
     int chunk = 0;           // edges per chunk

@@ -48,11 +48,8 @@ static void launch_nf(const MainParams& q0, unsigned blocks, int sdepth, size_t 
         if (evs) cudaEventRecord(evs->start[1], side);
         q.ray_counter = rc ? rc + 1 : nullptr;
         const size_t bytes = split_stack + kSplitWarps * sizeof(ReflShared<NF>) + size_t(kSplitWarps) * 32 * NF * 3 * 4;
-        static bool attr = false;
-        if (!attr) {
-            cudaFuncSetAttribute(k_reflect<T, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            attr = true;
-        }
+        static std::atomic<unsigned long long> raised{0};
+        raise_shared_limit((const void*)k_reflect<T, NF>, 200 * 1024, raised);
         k_reflect<T, NF><<<grid, kSplitBlock, bytes, side>>>(q, sdepth, tw);
         note_launch();
         if (evs) cudaEventRecord(evs->end[1], side);
@@ -68,12 +65,9 @@ static void launch_nf(const MainParams& q0, unsigned blocks, int sdepth, size_t 
     if ((c & 4) && dp.chunks > 0) {
         q.ray_counter = rc ? rc + 2 : nullptr;
         const size_t bytes = kSplitWarps * sizeof(DiffShared<NF>) + size_t(kSplitWarps) * 32 * NF * 9 * 4;
-        static bool attr = false;
-        if (!attr) {
-            cudaFuncSetAttribute(k_diffract_vis<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            cudaFuncSetAttribute(k_diffract_utd<T, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            attr = true;
-        }
+        static std::atomic<unsigned long long> raised_vis{0}, raised_utd{0};
+        raise_shared_limit((const void*)k_diffract_vis<T>, 200 * 1024, raised_vis);
+        raise_shared_limit((const void*)k_diffract_utd<T, NF>, 200 * 1024, raised_utd);
         for (int k = 0; k < dp.chunks; ++k) {
             const int j0 = k * dp.chunk;
             if (dp.run_vis) {
