@@ -935,7 +935,7 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
     const V3<T> ST = cast3<T>(S);
     const V3<float> Rf = active ? rx_point(p, r) : v3(0.f, 0.f, 0.f);
     const V3<double> R = cast3<double>(Rf);
-    unsigned rays = 0, searches = 0, closed_pairs = 0;  // of one thread: at most 2 per edge of the list
+    unsigned long long rays = 0;
     __shared__ TileBounds all_bounds[kSplitWarps];
     __shared__ int all_open[kSplitWarps * kEdgeSpan], all_n[kSplitWarps];
     TileBounds& bounds = all_bounds[grp.index];
@@ -965,7 +965,6 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
                 const int mine = next + __popc(idle & lanemask_lt());
                 if (jt < 0 && mine < end) {
                     jt = mine;
-                    ++searches;
                     const V3<float> near_end = edge_shaft(sc, list[jt], S, bounds, sh, ig);
                     q.start(sc, near_end, v3(0.5f * (bounds.lo[0] + bounds.hi[0]), 0.5f * (bounds.lo[1] + bounds.hi[1]),
                                              0.5f * (bounds.lo[2] + bounds.hi[2])));
@@ -987,13 +986,20 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
                 else if (q.next != ShaftSearch::kNone) q.node(sc, stack);
                 if (closed) {
                     vis_words[tile * chunk + (jt - j0)] = 0u;
-                    ++closed_pairs;
                 } else if (q.done()) open_edges[atomicAdd(&num_open, 1)] = jt;
                 if (closed || q.done()) jt = -1;
             }
         }
         grp.sync();
         const int n = num_open;
+        if (p.ray_counter && p.freq_base == 0 && grp.rank == 0) {
+            // a closed pair answers one query of each cell; every pair was searched once
+            const int pairs = min(jend - jb, width), cells = __popc(__ballot_sync(kFull, active));
+            if (lane == 0) {
+                atomicAdd(p.ray_counter + 1, (unsigned long long)(pairs - n) * cells);
+                atomicAdd(p.ray_counter + 2, (unsigned long long)pairs);
+            }
+        }
         for (int i = grp.rank; i < n; i += grp.warps) {
             const int j = open_edges[i];
             bool vis = false;
@@ -1027,12 +1033,7 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_diffract_vis(MainParams p, i
         }
         grp.sync();
     }
-    if (p.ray_counter && p.freq_base == 0) {
-        const int cells = __popc(__ballot_sync(kFull, active));  // a closed pair answers one query of each
-        if (rays) atomicAdd(p.ray_counter, (unsigned long long)rays);
-        if (closed_pairs) atomicAdd(p.ray_counter + 1, (unsigned long long)closed_pairs * cells);
-        if (searches) atomicAdd(p.ray_counter + 2, (unsigned long long)searches);
-    }
+    if (p.ray_counter && p.freq_base == 0 && rays) atomicAdd(p.ray_counter, rays);
 }
 
 // UTD fields of the visible pairs of edges [j0, j0 + chunk).  The tile's
