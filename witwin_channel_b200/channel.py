@@ -5,8 +5,8 @@ Same definitions as the reference's ``PathResult.cir`` / ``.cfr`` / ``.taps``
 deterministic ``PathTable`` (records in canonical (rx, tx) order): delays are
 normalised per link by their minimum, the coefficient is the powered path
 field, and the CFR is H(f_k) = sum_p a_p exp(-j 2 pi tau_p f_k).  The CFR runs
-in ``libwcb200.so`` (``wcb_cfr``), one warp per link, each link's spectrum
-written once.
+in ``libwcb200.so`` (``wcb_cfr_guarded``), two warps per link, each link's
+spectrum written once.
 """
 
 from __future__ import annotations

@@ -21,8 +21,8 @@ namespace wcb {
 
 constexpr int kWarpsPerBlock = 4;              // LoS/transmission: one tile per warp
 constexpr int kCompBlock = kWarpsPerBlock * 32;
-constexpr int kSplitWarps = 8;                 // reflection/diffraction: one tile per block,
-constexpr int kSplitBlock = kSplitWarps * 32;  // its candidates interleaved over 8 warps
+constexpr int kSplitWarps = 8;                 // reflection/diffraction: 1, 2 or 4 tiles per block,
+constexpr int kSplitBlock = kSplitWarps * 32;  // a tile's candidates dealt over its 8, 4 or 2 warps
 constexpr int kQueueCap = 64;
 constexpr int kEdgeSpan = 128;   // diffraction edges per warp between two lists of open pairs
 constexpr int kEdgeRefill = 8;   // idle lanes that take new edges
@@ -469,9 +469,9 @@ WCB_D int queue_pop_faces(int* q, int* qfaces, int size, int n, int lane) {
 // and leave after one traversal instead of idling while a visible path of
 // the same batch traces its remaining segments and its field.
 //
-// Bound by instruction issue and fetch (ncu on the 64-box canyon, 256^2 cells:
-// 32 % issue, 4.1 no-instruction stalls per issue; DRAM below 1 %).  Most of
-// the work was on candidates that no receiver of a tile has: of 1.71 M (tile,
+// Bound by instruction issue and the wait for a block's other tiles (ncu on the
+// 64-box canyon, 256^2 cells: 42 % issue, 3.8 barrier, 2.2 wait and 1.9
+// no-instruction stalls per issue; DRAM below 1 %).  Most of the work was on candidates that no receiver of a tile has: of 1.71 M (tile,
 // candidate) pairs the last bounce's box alone left 222 k (6.7 M FP64 back
 // projections), all bounces' boxes leave 61 k and the blocked last legs 31 k
 // (0.77 M).  Testing the receiver's leg first takes the visibility segments of
@@ -628,7 +628,8 @@ __global__ void __launch_bounds__(kSplitBlock, sizeof(T) == 4 ? 3 : 2) k_reflect
     };
 
     // stage A: FP64 back projection + containment for up to 32 items; the
-    // survivors enter queue B at segment 0
+    // survivors enter queue B at segment d (last hit -> receiver), which stage B
+    // counts down; a path is visible after segment 0
     auto process_a = [&](int n) __attribute__((always_inline)) {
         int it_lane = 0, c = 0, d = 1;
         if (lane < n) {
@@ -901,7 +902,7 @@ WCB_D V3<float> edge_shaft(const SceneDev& sc, int edge, V3<double> S, const Til
 // for that lane's cell, Q the clamped stationary point on the edge moved by
 // kDiffractionRayBias along its exterior bisector.
 //
-// Issue bound (68-78 %).  One thread first tries to close a whole (tile, edge)
+// Issue bound (ncu: 61 % on the canyon, 78 % on the 2048-box city).  One thread first tries to close a whole (tile, edge)
 // pair with one triangle (shaft.cuh), so a warp settles 32 pairs with one
 // divergent traversal where it took 32 coherent ones; only open pairs are
 // traced per cell, the receiver's leg first (49 % of the canyon's are clear,

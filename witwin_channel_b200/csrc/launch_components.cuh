@@ -18,7 +18,10 @@ namespace wcb {
 // 7.3 at 1 (whole call).  The UTD kernel, whose batches are dealt out evenly,
 // wants more: 0.34 at 4 and 0.25 at 8 on the canyon (2,048 tiles), the same at 1
 // and 2 on the city.  FP64 keeps eight: its warps' sums are rounded to FP32 before
-// they are added, so another grouping would be another result.
+// they are added, so another grouping would be another result.  In mixed precision
+// the grouping, and with it the rounding of a cell's sum, follows the tile count of
+// the whole call: a shard or a single transmitter of a larger map agrees with that
+// map to FP32 rounding, not bit for bit.
 template <typename T>
 static int trace_tile_warps(long long tiles) {
     if (sizeof(T) == 8) return 8;

@@ -378,7 +378,8 @@ static long long vis_word_budget() {
 // tile tests decide per receiver, one candidate or edge per thread, and 32 times
 // as many warps share the work.  37 receivers among 16 boxes, one B200:
 // k_reflect 0.60 -> 0.13 ms and k_diffract_vis 0.10 -> below 0.04 ms.  FP64 sums a
-// tile's fields in shares whose rounding depends on the tile, and keeps 32.
+// tile's fields in shares whose rounding depends on the tile, and keeps 32; mixed
+// sums on either side of the line agree to FP32 rounding.
 constexpr long long kSingleCellTiles = 2048;
 
 static int tile_cells(const wcb_solve_desc& d) {

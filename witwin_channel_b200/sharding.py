@@ -3,7 +3,9 @@
 The units of the deterministic solve (transmitter, frequency, receiver tile)
 are independent: each rank owns a disjoint slice of them, solves it with no
 collective on the data path, and the per-rank outputs are joined by
-concatenation.  The only collectives are the step-time reduction (max over
+concatenation.  Paths and FP64 maps do not depend on the split; a mixed
+precision map's cells are summed in an order that follows the size of the
+call, so a joined map agrees with an unsplit one to FP32 rounding.  The only collectives are the step-time reduction (max over
 ranks) and, when a caller wants the whole map on every rank, one all-gather
 of the outputs at the end.  A gradient step over a sharded job (a loss that
 is a sum over the ranks' cells) needs one exchange: the sum of the ranks'
