@@ -819,6 +819,8 @@ def _large_run(device, steps: int = 2) -> dict:
         "rays": rays,
         "rays_traced": prof["rays_traced"] + prof["prep_rays"],
         "rays_per_s_kernels": rays / ((prof["main_ms"] + prof["prep_ms"]) / 1000.0),
+        "rays_traced_per_s_kernels": (prof["rays_traced"] + prof["prep_rays"])
+        / ((prof["main_ms"] + prof["prep_ms"]) / 1000.0),
         "paths": int(res.metadata["counts"]["path_count"]),
         "cfr_ms": cfr_ms,
         "cfr_bytes": int(h.numel() * 8),
